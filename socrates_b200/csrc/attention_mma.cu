@@ -256,6 +256,7 @@ attn_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float* __
         }
     }
 
+    const WholeTileCopy<D, KTD, NTHR> copy(kbuf, vbuf, KTD * D, k_pool, v_pool, bs_log2, Hkv, kh);
     ColState<D, NBQ> st;
     st.init();
     uint32_t qf[D / 16][4];
@@ -272,12 +273,15 @@ attn_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float* __
         const int buf = i % S;
         const int ts = (tile_begin + i) * KTD;
         const bool masked = ts < k_begin || ts + KTD > k_end;       // only the partition's edge tiles
-        // tile nxt's copies go out in four doses between the phases of tile i (slot (i-1)%S is free)
+        // tile nxt's copies go out in four doses between the phases of tile i (slot (i-1)%S is free), or, where it
+        // lies at an edge of the partition, at once
+        const int nxt_ts = (tile_begin + nxt) * KTD;
+        const bool doses = nxt < n_tiles && nxt_ts >= k_begin && nxt_ts + KTD <= k_end;
+        if (nxt < n_tiles && !doses)
+            load_kv_tile<D, KTD, NTHR>(kbuf + (nxt % S) * KTD * D, vbuf + (nxt % S) * KTD * D, k_pool, v_pool, stab, pg_begin,
+                                       bs_log2, Hkv, kh, nxt_ts, k_begin, k_end);
         auto between = [&](int part) {
-            if (nxt < n_tiles)
-                load_kv_tile_part<D, KTD, NTHR>(part, kbuf + (nxt % S) * KTD * D, vbuf + (nxt % S) * KTD * D, k_pool,
-                                                v_pool, stab, pg_begin, bs_log2, Hkv, kh, (tile_begin + nxt) * KTD,
-                                                k_begin, k_end);
+            if (doses) copy.dose(part, nxt % S, stab - pg_begin, nxt_ts);
         };
         if constexpr (MAPPED)
             warp_tile_decode<D, NBQ>(st, qf, kbuf + buf * KTD * D, vbuf + buf * KTD * D, warp * 16, ts, pos, k_begin,

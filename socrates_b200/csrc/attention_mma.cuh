@@ -96,37 +96,51 @@ __device__ __forceinline__ void load_kv_tile(bf16* ks, bf16* vs, const bf16* __r
     }
 }
 
-// Quarter `part` (0..3) of load_kv_tile's copies: the decode kernel issues a tile's copies in
-// four doses between the phases of the tile before it.  Sixteen cp.async per thread in one
-// burst, from every warp of the SM at the same moment after the block's barrier, queue up in
-// the load/store unit: a warp then sat 1,500 clocks of a 3,400-clock tile in that burst.
-template <int D, int KTILE, int NTHR>
-__device__ __forceinline__ void load_kv_tile_part(int part, bf16* ks, bf16* vs, const bf16* __restrict__ k_pool,
-                                                  const bf16* __restrict__ v_pool, const int* table, int table_base,
-                                                  int bs_log2, int Hkv, int kh, int tile_start, int lo, int hi) {
-    constexpr int CH = D / 8;
-    constexpr int ROWS = NTHR / CH;
-    constexpr int IT = KTILE / ROWS;                // copies of one thread per tile and pool
+// The copies of a tile whose keys are ALL wanted, in four doses that the decode kernels issue between the phases of the
+// tile before it.  Sixteen cp.async per thread in one burst, from every warp of the SM at the same moment after the
+// block's barrier, queue up in the load/store unit: a warp then sat 1,500 clocks of a 3,400-clock tile in that burst.
+// What a pair of copies costs is a page number from shared memory, two multiply-adds and an addition: nothing is
+// compared with the ends of the range (tiles at an edge go through load_kv_tile), and the places in shared memory differ
+// by constants.  The decode kernels are bound by their instruction streams (8 warps an SM), so this is time: in the
+// split-key kernel, 8 rows of 4,096 keys (32 query and 8 KV heads of 128) 28.0 -> 25.2 us, 64 rows of 2,048 keys
+// 94 -> 87 us (537 MB: 6.2 TB/s).
+template <int D, int KTILE, int NTHR> struct WholeTileCopy {
+    static constexpr int CH = D / 8;                // 16-byte columns of a row
+    static constexpr int ROWS = NTHR / CH;          // rows served per pass
+    static constexpr int IT = KTILE / ROWS;         // copies of one thread per tile and pool
     static_assert(NTHR % CH == 0 && KTILE % ROWS == 0, "threads must tile the tile");
-    const int c = threadIdx.x % CH;
-    const int r0 = threadIdx.x / CH;
-    const int bs_mask = (1 << bs_log2) - 1;
-#pragma unroll
-    for (int it = 0; it < IT; ++it) {
-        if (it * 4 / IT != part) continue;          // dose `part` holds the copies it with it*4/IT == part
-        const int key = r0 + it * ROWS;
-        const int pos = tile_start + key;
-        const bool valid = pos >= lo && pos < hi;
-        size_t src = 0;
-        if (valid) {
-            const int page = table[(pos >> bs_log2) - table_base];
-            src = ((((size_t)page * Hkv + kh) << bs_log2) + (pos & bs_mask)) * D + c * 8;
-        }
-        const int off = tile_off<D>(key, c);
-        cp_async16(smem_u32(ks + off), k_pool + src, valid ? 16 : 0);
-        cp_async16(smem_u32(vs + off), v_pool + src, valid ? 16 : 0);
+    static_assert(ROWS % 8 == 0, "the rows of a thread share their swizzle");
+    const char* k_thread;
+    long long to_v;                                 // bytes from a key to its value
+    int page_bytes, bs_log2, bs_mask, r0;
+    uint32_t k_dst, v_dst;
+    int stage_bytes;
+    // `ks`, `vs`: stage 0; `stage_elems` between stages
+    __device__ __forceinline__ WholeTileCopy(const bf16* ks, const bf16* vs, int stage_elems, const bf16* k_pool,
+                                             const bf16* v_pool, int bs_log2_, int Hkv, int kh) {
+        const int c = threadIdx.x % CH;
+        r0 = threadIdx.x / CH;
+        bs_log2 = bs_log2_;
+        bs_mask = (1 << bs_log2) - 1;
+        k_thread = reinterpret_cast<const char*>(k_pool + (((size_t)kh << bs_log2) * D + c * 8));
+        to_v = reinterpret_cast<const char*>(v_pool) - reinterpret_cast<const char*>(k_pool);
+        page_bytes = (Hkv << bs_log2) * D * 2;
+        k_dst = smem_u32(ks + tile_off<D>(r0, c));
+        v_dst = smem_u32(vs + tile_off<D>(r0, c));
+        stage_bytes = stage_elems * 2;
     }
-}
+    // `pages[pos >> bs_log2]` is the physical page of position pos
+    __device__ __forceinline__ void dose(int part, int stage, const int* pages, int tile_start) const {
+#pragma unroll
+        for (int it = 0; it < IT; ++it) {
+            if (it * 4 / IT != part) continue;      // dose `part` holds the copies it with it*4/IT == part
+            const int pos = tile_start + r0 + it * ROWS;
+            const char* src = k_thread + (long long)pages[pos >> bs_log2] * page_bytes + (pos & bs_mask) * (D * 2);
+            cp_async16(k_dst + stage * stage_bytes + it * (ROWS * D * 2), src, 16);
+            cp_async16(v_dst + stage * stage_bytes + it * (ROWS * D * 2), src + to_v, 16);
+        }
+    }
+};
 
 // State of the two accumulator rows a thread owns (rows lane/4 and lane/4 + 8 of the
 // warp's 16): running maximum (raw scores), this thread's share of the running sum, and
