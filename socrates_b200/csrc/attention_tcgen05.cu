@@ -201,7 +201,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_k, const __g
                             const int* __restrict__ seq_first_pos, int R, int Hq, int Hkv, int BS, int window,
                             float scale_log2, int* __restrict__ status, const bf16* __restrict__ gate,
                             long long gate_stride, int gate_per_dim, int has_sink, float sink_raw, int keep_first,
-                            float* __restrict__ out_f32, ScoreMap map) {
+                            float* __restrict__ out_f32, int skip_single, ScoreMap map) {
     constexpr int PANELS = D / 64;                         // 64-dim panels of 128-byte rows
     constexpr int PANEL_Q = ROWS * 128;                    // bytes of one Q panel
     constexpr int PANEL_KV = KTILE * 128;                  // bytes of one K or V panel
@@ -255,7 +255,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_k, const __g
     int tile = gridDim.x / Hkv - 1 - blockIdx.x / Hkv, r = 0, t0 = 0, n_tok = 0;
     for (; r < R; ++r) {
         const int a = seq_starts[r], len = seq_starts[r + 1] - a;
-        const int tiles = (len + TQ - 1) / TQ;
+        const int tiles = skip_single && len == 1 ? 0 : (len + TQ - 1) / TQ;
         if (tile < tiles) {
             t0 = a + tile * TQ;
             n_tok = min(TQ, len - tile * TQ);
@@ -650,8 +650,8 @@ template <int D, int MAPPED>
 int launch(const CUtensorMap& mk, const CUtensorMap& mv, void* out, const void* q, const int* block_table,
            int table_width, const int* seq_starts, const int* seq_rows, const int* seq_first_pos, int R, int N,
            int Hq, int Hkv, int BS, int window, float scale, int* status, const void* gate, long long gate_stride,
-           int gate_per_dim, int has_sink, float sink, int keep_first, float* out_f32, const ScoreMap& map,
-           cudaStream_t stream) {
+           int gate_per_dim, int has_sink, float sink, int keep_first, float* out_f32, int skip_single,
+           const ScoreMap& map, cudaStream_t stream) {
     auto kernel = attn_prefill_tcgen05_kernel<D, MAPPED>;
     static sb::OncePerDevice once_per_device;
     bool& configured = once_per_device.flag();
@@ -666,7 +666,7 @@ int launch(const CUtensorMap& mk, const CUtensorMap& mv, void* out, const void* 
     sb::launch(kernel, grid, dim3(THREADS), smem_bytes<D>() + table_width * 4, stream, mk, mv, (bf16*)out,
                (const bf16*)q, block_table, table_width, seq_starts, seq_rows, seq_first_pos, R, Hq, Hkv, BS, window,
                MAPPED != 0 ? scale : scale * LOG2E, status, (const bf16*)gate, gate_stride, gate_per_dim, has_sink,
-               has_sink ? (MAPPED != 0 ? sink * LOG2E : sink / scale) : 0.f, keep_first, out_f32, map);
+               has_sink ? (MAPPED != 0 ? sink * LOG2E : sink / scale) : 0.f, keep_first, out_f32, skip_single, map);
     return 0;
 }
 
@@ -685,7 +685,8 @@ extern "C" int sb_attention_tcgen05_supports(int Hq, int Hkv, int D, int page_si
 // (`gate` [N, gate_stride] bfloat16, one column per head, or per head and dim) and a sink (a score
 // whose exponential joins the denominator without a value); `keep_first`: a window also sees the first
 // so many keys of its row; `out_f32` (float32 [N, Hq*D], or null): the rows are written there unrounded
-// and ungated instead of to `out`; `cap`, `slopes` [Hq] and `chunk` as in score_map.cuh (0 / null: none).
+// and ungated instead of to `out`; `cap`, `slopes` [Hq] and `chunk` as in score_map.cuh (0 / null: none);
+// `skip_single`: requests that bring one token are left out (their rows of the output are not written).
 extern "C" int sb_attention_prefill_tcgen05(void* out, const void* q, const void* k_pool, const void* v_pool,
                                             int num_pages, const int* block_table, int table_width,
                                             const int* seq_starts, const int* seq_rows,
@@ -693,7 +694,7 @@ extern "C" int sb_attention_prefill_tcgen05(void* out, const void* q, const void
                                             int page_size, int window, float scale, int* status,
                                             const void* gate, long long gate_stride, int gate_per_dim, int has_sink,
                                             float sink, int keep_first, float* out_f32, float cap, const float* slopes,
-                                            int chunk, cudaStream_t stream) {
+                                            int chunk, int skip_single, cudaStream_t stream) {
     SB_REQUIRE(cap >= 0.f && chunk >= 0 && !(chunk > 0 && window > 0),
                "attention_tcgen05: a cap of %f, chunks of %d beside a window of %d", (double)cap, chunk, window);
     SB_REQUIRE(keep_first >= 0, "attention_tcgen05: %d kept keys", keep_first);
@@ -716,7 +717,7 @@ extern "C" int sb_attention_prefill_tcgen05(void* out, const void* q, const void
 #define SB_TILE(D_, MAPPED_) \
     launch<D_, MAPPED_>(mk, mv, out, q, block_table, table_width, seq_starts, seq_rows, seq_first_pos, R, N, Hq, Hkv, \
                         page_size, window, scale, status, gate, gate_stride, gate_per_dim, has_sink, sink, keep_first, \
-                        out_f32, map, stream)
+                        out_f32, skip_single, map, stream)
     int rc;
     if (cap > 0.f && cap * LOG2E <= BOUND_LOG2 && !has_sink) rc = D == 64 ? SB_TILE(64, 2) : SB_TILE(128, 2);
     else if (map.maps_scores()) rc = D == 64 ? SB_TILE(64, 1) : SB_TILE(128, 1);

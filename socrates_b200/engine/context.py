@@ -111,7 +111,8 @@ class StepContext:
     def __init__(self, dtype: torch.dtype, device, buffers: Buffers, num_tokens: int, num_seqs: int,
                  token_ids, positions, token_rows, seq_starts, seq_rows, seq_first_pos, logit_index,
                  all_decode: bool, max_context: int, host_batch=None, num_sms: int = 148,
-                 status: Optional[torch.Tensor] = None, token_feedback: Optional[torch.Tensor] = None):
+                 status: Optional[torch.Tensor] = None, token_feedback: Optional[torch.Tensor] = None,
+                 share_keys: bool = False):
         self.dtype, self.device, self.buffers = dtype, device, buffers
         self.num_tokens, self.num_seqs = num_tokens, num_seqs
         self.token_ids, self.positions, self.token_rows = token_ids, positions, token_rows
@@ -120,6 +121,9 @@ class StepContext:
         self.all_decode = all_decode        # every request brings exactly one token
         self.max_context = max_context      # upper bound of any request's length after this step
         self.host_batch = host_batch        # the host-side entries; None while a graph is recorded
+        self.share_keys = share_keys        # a decode step whose rows differ much (see Model.prefers_shares)
+        # keys of the longest request that brings one token (0: there is none, or the step is being recorded)
+        self.longest_single = max((e.start + 1 for e in host_batch or () if len(e.tokens) == 1), default=0)
         self.num_sms = num_sms
         self.status = status                # int32 device word the tensor-core kernels report to
         self.token_feedback = token_feedback   # int32 device tokens that ids -1 - j stand for (see ops.embed)

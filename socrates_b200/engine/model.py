@@ -40,6 +40,12 @@ class Model:
         # programmatic dependent launch): `serial_launches = True` on the part.
         self.dependent_launch = not any(getattr(p, "serial_launches", False)
                                         for layer in self.layers for p in getattr(layer, "parts", list)())
+        dealers = {}
+        for layer in self.layers:
+            for p in getattr(layer, "parts", list)():
+                if hasattr(p, "prefers_shares"):
+                    dealers.setdefault((p.Hq, p.Hkv, p.D, p.window), p)
+        self._key_dealers = list(dealers.values())
         self.final_norm = build_part("norm", plan.final_norm, plan.final_norm.name)
         self.head = build_part("head", plan.head, plan.head.name)
         self.dtype: Optional[torch.dtype] = None
@@ -89,6 +95,11 @@ class Model:
     def supports_graph(self) -> bool:
         return (all(l.supports_graph for l in self.layers)
                 and all(getattr(op, "supports_graph", True) for op in self.stream_ops.values()))
+
+    def prefers_shares(self, lengths, num_sms: int) -> bool:
+        """Whether a decode step over rows of so many keys should deal the keys of all rows to the GPU's blocks in equal
+        shares (parts say so through an optional `prefers_shares`; asked once for layers of one shape)."""
+        return any(p.prefers_shares(lengths, num_sms) for p in self._key_dealers)
 
     # ------------------------------------------------------------------ one step
     def forward(self, ctx: StepContext, cache) -> torch.Tensor:

@@ -98,13 +98,14 @@ class ModelRunner:
         self.sample_scratch = torch.zeros(ops.sample_scratch_size(max_tokens, self.vocab), dtype=torch.int32,
                                           device=self.device)
         self.use_graphs = use_graphs and model.supports_graph
-        self._graphs: Dict[Tuple[int, int, bool], Tuple[torch.cuda.CUDAGraph, Optional[torch.Tensor]]] = {}
+        # by (rows, whether tokens are drawn, whether keys are dealt in shares)
+        self._graphs: Dict[Tuple[int, bool, bool], Tuple[torch.cuda.CUDAGraph, Optional[torch.Tensor]]] = {}
         self._eager_decode_done: set = set()
         self.num_sms = torch.cuda.get_device_properties(self.device).multi_processor_count
         self.steps_run = 0
         self.graph_replays = 0
         self.kernel_launches = 0    # kernels launched by steps, replays of recorded graphs included
-        self._graph_kernels: Dict[Tuple[int, bool], int] = {}
+        self._graph_kernels: Dict[Tuple[int, bool, bool], int] = {}
 
     # ------------------------------------------------------------------ staging
     def _stage(self) -> Tuple[torch.Tensor, int]:
@@ -185,7 +186,8 @@ class ModelRunner:
         self._staging[slot][1] = ev
         return N, M, R, all_decode, max_ctx
 
-    def _context(self, N: int, M: int, R: int, all_decode: bool, max_ctx: int, host_batch) -> StepContext:
+    def _context(self, N: int, M: int, R: int, all_decode: bool, max_ctx: int, host_batch,
+                 share_keys: bool = False) -> StepContext:
         L, m = self.layout, self.dev_meta
         return StepContext(
             self.dtype, self.device, self.buffers, N, R,
@@ -194,7 +196,7 @@ class ModelRunner:
             seq_first_pos=m[L.seq_first:L.seq_first + R],
             logit_index=m[L.logit:L.logit + M] if M else None,
             all_decode=all_decode, max_context=max_ctx, host_batch=host_batch, num_sms=self.num_sms,
-            status=self.status, token_feedback=self.sampled)
+            status=self.status, token_feedback=self.sampled, share_keys=share_keys)
 
     def begin_read(self, count: int) -> Tuple[int, int]:
         """Start the copy of the `count` tokens the last step sampled (and of the kernels'
@@ -229,34 +231,41 @@ class ModelRunner:
         number of graphs recorded."""
         if not self.use_graphs:
             return 0
-        L, made = self.layout, 0
+        made = 0
         for n in range(1, min(max_width, self.max_seqs, self.cache.max_rows) + 1):
-            key = (n, sample)
-            if key in self._graphs:
-                continue
-            buf, slot = self._stage()
-            nb = self._staging_np[slot]
-            nb[:] = 0
-            nb[L.rows:L.rows + n] = list(range(n))
-            nb[L.logit:L.logit + n] = list(range(n))
-            nb[L.seq_starts:L.seq_starts + n + 1] = list(range(n + 1))
-            nb[L.seq_rows:L.seq_rows + n] = list(range(n))
-            self.dev_meta.copy_(buf, non_blocking=True)
-            ev = self._events[slot]
-            ev.record()
-            self._staging[slot][1] = ev
-            ctx = self._context(n, n, n, True, self.cache.max_len, None)
-            self._run(ctx, n, sample)                       # loads every kernel, sizes every buffer
-            graph = torch.cuda.CUDAGraph()
-            before = Counters.launches
-            with torch.cuda.graph(graph):
-                logits, tokens = self._run(ctx, n, sample)
-            self._graph_kernels[key] = Counters.launches - before
-            self._graphs[key] = (graph, logits, tokens)
-            self._eager_decode_done.add(key)
-            made += 1
+            # one long row among short ones: could this width ever deal its keys in shares?
+            uneven = (self.dtype == torch.bfloat16
+                      and self.model.prefers_shares([self.cache.max_len] + [1] * (n - 1), self.num_sms))
+            made += sum(self._record_width(n, sample, share) for share in ((False, True) if uneven else (False,)))
         torch.cuda.synchronize()
         return made
+
+    def _record_width(self, n: int, sample: bool, share: bool) -> int:
+        """Record one decode graph (see warmup); returns how many were recorded."""
+        L, key = self.layout, (n, sample, share)
+        if key in self._graphs:
+            return 0
+        buf, slot = self._stage()
+        nb = self._staging_np[slot]
+        nb[:] = 0
+        nb[L.rows:L.rows + n] = list(range(n))
+        nb[L.logit:L.logit + n] = list(range(n))
+        nb[L.seq_starts:L.seq_starts + n + 1] = list(range(n + 1))
+        nb[L.seq_rows:L.seq_rows + n] = list(range(n))
+        self.dev_meta.copy_(buf, non_blocking=True)
+        ev = self._events[slot]
+        ev.record()
+        self._staging[slot][1] = ev
+        ctx = self._context(n, n, n, True, self.cache.max_len, None, share)
+        self._run(ctx, n, sample)                       # loads every kernel, sizes every buffer
+        graph = torch.cuda.CUDAGraph()
+        before = Counters.launches
+        with torch.cuda.graph(graph):
+            logits, tokens = self._run(ctx, n, sample)
+        self._graph_kernels[key] = Counters.launches - before
+        self._graphs[key] = (graph, logits, tokens)
+        self._eager_decode_done.add(key)
+        return 1
 
     def check_status(self) -> None:
         """Raise if a kernel reported that one of its bounded waits gave up.  Reads one
@@ -299,11 +308,14 @@ class ModelRunner:
         self.cache.flush()
         N, M, R, all_decode, max_ctx = self._fill(entries, sampling, ahead)
         sample = sampling is not None
+        # decoding rows of very different lengths go through another attention kernel (and a graph of their own)
+        share = (all_decode and self.dtype == torch.bfloat16
+                 and self.model.prefers_shares([e.start + 1 for e in entries], self.num_sms))
         self.steps_run += 1
         if self.use_graphs and all_decode and M == N:
-            key = (N, sample)
+            key = (N, sample, share)
             if key not in self._graphs and key in self._eager_decode_done:
-                ctx = self._context(N, M, R, True, self.cache.max_len, None)
+                ctx = self._context(N, M, R, True, self.cache.max_len, None, share)
                 graph = torch.cuda.CUDAGraph()
                 before = Counters.launches
                 with torch.cuda.graph(graph):
@@ -318,7 +330,7 @@ class ModelRunner:
                 return StepResult(logits, tokens, N)
             self._eager_decode_done.add(key)
             max_ctx = self.cache.max_len     # the same launch shapes the graph will record
-        ctx = self._context(N, M, R, all_decode, max_ctx, entries)
+        ctx = self._context(N, M, R, all_decode, max_ctx, entries, share)
         before = Counters.launches
         logits, tokens = self._run(ctx, M, sample)
         self.kernel_launches += Counters.launches - before

@@ -468,6 +468,52 @@ def attention_decode_stream(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Te
         "attention_decode_stream")
 
 
+def attention_balanced_supports(num_heads: int, num_kv_heads: int, head_dim: int, page_size: int, requests: int) -> bool:
+    """Whether the equal-shares decode kernel takes this shape (bfloat16) in a step of `requests` requests."""
+    return bool(library().sb_attention_balanced_supports(num_heads, num_kv_heads, head_dim, page_size, requests))
+
+
+def attention_balanced_shares(num_heads: int, num_kv_heads: int, head_dim: int, requests: int, num_sms: int) -> int:
+    """Shares the equal-shares decode kernel cuts each KV head's keys into."""
+    return library().sb_attention_balanced_shares(num_heads, num_kv_heads, head_dim, requests, num_sms)
+
+
+def attention_decode_balanced(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
+                              block_table: torch.Tensor, seq_starts: torch.Tensor, seq_rows: torch.Tensor,
+                              seq_first_pos: torch.Tensor, num_heads: int, scale: float, window: int, shares: int,
+                              part_o: torch.Tensor, part_ml: torch.Tensor, counters: torch.Tensor) -> None:
+    """Paged attention (bfloat16) of the requests of a step that bring ONE token, their keys dealt to the
+    blocks in `shares` equal shares per KV head; rows of `out` that belong to other requests are left alone.
+
+    Scratch: part_o float32 with Hq*shares*2*D elements, part_ml with Hq*shares*2*2, and int32 `counters`
+    with R*Hkv entries that are zero before the first call (the kernel leaves them zero).
+
+    The kernel reads the block table, offsets, rows, positions and the keys and values below each position
+    before it waits for the kernel that precedes it on the stream: those must be older than that kernel (a
+    host copy, an earlier step)."""
+    N = q.shape[0]
+    _, Hkv, BS, D = k_pool.shape
+    Hq, R = num_heads, seq_rows.numel()
+    _want(q, "q", torch.bfloat16, (N, Hq * D))
+    _want(out, "out", torch.bfloat16, (N, Hq * D))
+    _want(k_pool, "k_pool", torch.bfloat16)
+    _want(v_pool, "v_pool", torch.bfloat16, k_pool.shape)
+    _want(block_table, "block_table", torch.int32)
+    _want(seq_starts, "seq_starts", torch.int32, (R + 1,))
+    _want(seq_rows, "seq_rows", torch.int32, (R,))
+    _want(seq_first_pos, "seq_first_pos", torch.int32, (R,))
+    _want(part_o, "part_o", torch.float32)
+    _want(part_ml, "part_ml", torch.float32)
+    _want(counters, "counters", torch.int32)
+    if (part_o.numel() < Hq * shares * 2 * D or part_ml.numel() < Hq * shares * 2 * 2 or counters.numel() < R * Hkv):
+        raise KernelError("attention scratch buffers are too small")
+    lib = library()
+    check(lib, lib.sb_attention_balanced(
+        _ptr(out), _ptr(part_o), _ptr(part_ml), _ptr(counters), _ptr(q), _ptr(k_pool), _ptr(v_pool),
+        _ptr(block_table), block_table.shape[1], _ptr(seq_starts), _ptr(seq_rows), _ptr(seq_first_pos), R, Hq, Hkv, D,
+        BS, int(window), float(scale), int(shares), _stream()), "attention_decode_balanced")
+
+
 def attention_decode_mma_blocks_per_sm(head_dim: int, variant: int = 0) -> int:
     """Blocks of the decode attention kernel that are resident on one SM at a time."""
     return library().sb_attention_decode_mma_blocks_per_sm(int(head_dim), int(variant))
@@ -484,13 +530,15 @@ def attention_prefill_tcgen05(out: torch.Tensor, q: torch.Tensor, k_pool: torch.
                               window: int = 0, gate: Optional[torch.Tensor] = None, gate_per_dim: bool = False,
                               sink: Optional[float] = None, keep_first: int = 0,
                               out_float: Optional[torch.Tensor] = None, softcap: float = 0.0,
-                              slopes: Optional[torch.Tensor] = None, chunk: int = 0) -> None:
+                              slopes: Optional[torch.Tensor] = None, chunk: int = 0,
+                              skip_single: bool = False) -> None:
     """Paged causal attention of prompt portions on tcgen05 (scores and P.V in tensor
     memory, pages brought in by TMA).  Arguments as `attention_prefill_mma`, plus the int32
     status word that receives a non-zero code if a bounded wait inside the kernel gave up.
     `keep_first`: a window also sees the first so many keys of its row.  `out_float` (float32
     [N, Hq*D]): the rows go there unrounded instead of to `out` (which may then be None).
-    `softcap`, `slopes`, `chunk` as in `attention_decode_mma`."""
+    `softcap`, `slopes`, `chunk` as in `attention_decode_mma`.  `skip_single`: requests that bring one
+    token are left out (see `attention_decode_balanced`); their rows of `out` are not written."""
     N = q.shape[0]
     pages, Hkv, BS, D = k_pool.shape
     R = seq_rows.numel()
@@ -517,7 +565,7 @@ def attention_prefill_tcgen05(out: torch.Tensor, q: torch.Tensor, k_pool: torch.
         _ptr(seq_starts), _ptr(seq_rows), _ptr(seq_first_pos), R, N, num_heads, Hkv, D, BS, int(window),
         float(scale), _ptr(status), _ptr(gate), gate_stride, int(gate_per_dim), int(sink is not None),
         float(sink or 0.0), int(keep_first), _ptr(out_float), float(softcap), _slopes(slopes, num_heads), int(chunk),
-        _stream()), "attention_prefill_tcgen05")
+        int(skip_single), _stream()), "attention_prefill_tcgen05")
 
 
 # ---------------------------------------------------------------------------------------------

@@ -16,7 +16,7 @@ portions and portions of prompts share a step with decode tokens.
 from __future__ import annotations
 
 import os
-from typing import Dict, Mapping, Optional
+from typing import Dict, Mapping, Optional, Sequence
 
 import torch
 
@@ -54,20 +54,41 @@ def decode_partitions(ctx, num_kv_heads: int, blocks_per_sm: int, keys_per_part:
     return parts
 
 
+# In a step that mixes prompt portions with decoding requests the tile kernel can serve both (a decoding request is a tile
+# of one token: its key tiles one after the other, 1.1 us each and more).  From this many keys in the longest such request
+# on, the decoding requests run in the equal-shares kernel beside it, one launch more.  Measured (8B shape, 12 layers, two
+# prompts of 511 beside 37 requests, ms a step, together / apart): 512 keys 6.10 / 6.29, 1,024: 6.46 / 6.39, 2,048: 7.03 /
+# 6.48, 4,096: 8.20 / 6.79.
+SINGLES_APART_FROM = 1024
+
+
+def balanced_attention(ctx, out, q, k_pool, v_pool, table, num_heads: int, scale: float, window: int) -> None:
+    """The step's requests of one token through the equal-shares decode kernel, with scratch of the step."""
+    Hkv, D, R = k_pool.shape[1], k_pool.shape[3], ctx.num_seqs
+    shares = ops.attention_balanced_shares(num_heads, Hkv, D, R, ctx.num_sms)
+    take = ctx.buffers.take_flat
+    ops.attention_decode_balanced(out, q, k_pool, v_pool, table, ctx.seq_starts, ctx.seq_rows, ctx.seq_first_pos,
+                                  num_heads, scale, window, shares,
+                                  take("attn_share_o", num_heads * shares * 2 * D, torch.float32),
+                                  take("attn_share_ml", num_heads * shares * 2 * 2, torch.float32),
+                                  take("attn_share_counters", ctx.buffers.max_rows * Hkv, torch.int32, zeroed=True))
+
+
 def paged_attention(ctx, out, q, k_pool, v_pool, table, num_heads: int, scale: float, window: int,
                     max_len: int) -> None:
     """Causal attention of every token of the step over its row's pages; this mixer's choice of kernel.
 
     bfloat16, a step in which every request brings one token (decode):
       * PAGED_PARTITION "auto": the split-key kernel (mma.sync), the partition COUNT chosen from
-        the batch width so that one wave of blocks fills the GPU.  Fastest; a request's numbers
-        differ in rounding with the width of the batch it is in.
+        the batch width so that one wave of blocks fills the GPU, or, where the rows' lengths differ so much
+        that the longest would run on alone (`prefers_shares`), the equal-shares kernel.  Fastest; a
+        request's numbers differ in rounding with the batch it is in.
       * PAGED_PARTITION = n: the streaming kernel over chunks of n keys at fixed key positions (the
         reference's meaning of the variable, model/kernels/csrc/paged_attention.cu:80-96; 0 = the
         whole row in one pass).  A request's numbers are the same bits alone and in a full batch;
         measured 12 to 25 % slower per decode step than "auto" on the 4B shape.
     bfloat16, other steps: the tile kernels (tcgen05 for head sizes 64 and 128, mma.sync for 16 and
-    32).  Everything else (the float32 engine above all): the SIMT kernel, whose split depends on
+    32); beside the tcgen05 kernel, decoding requests with long rows in the equal-shares kernel.  Everything else (the float32 engine above all): the SIMT kernel, whose split depends on
     `max_len` of the cache alone, so the float32 engine's numbers never depend on the batch.
     """
     Hkv, page_size, D = k_pool.shape[1], k_pool.shape[2], k_pool.shape[3]
@@ -75,8 +96,12 @@ def paged_attention(ctx, out, q, k_pool, v_pool, table, num_heads: int, scale: f
     bf16 = q.dtype == torch.bfloat16
     if bf16 and not ctx.all_decode:
         if ctx.status is not None and ops.attention_tcgen05_supports(num_heads, Hkv, D, page_size):
+            apart = (paged_partition() is None and ctx.longest_single >= SINGLES_APART_FROM
+                     and ops.attention_balanced_supports(num_heads, Hkv, D, page_size, ctx.num_seqs))
             ops.attention_prefill_tcgen05(out, q, k_pool, v_pool, table, ctx.seq_starts, ctx.seq_rows,
-                                          ctx.seq_first_pos, num_heads, scale, ctx.status, window)
+                                          ctx.seq_first_pos, num_heads, scale, ctx.status, window, skip_single=apart)
+            if apart:
+                balanced_attention(ctx, out, q, k_pool, v_pool, table, num_heads, scale, window)
             return
         if ops.attention_mma_supports(num_heads, Hkv, D, page_size, False):
             ops.attention_prefill_mma(out, q, k_pool, v_pool, table, ctx.seq_starts, ctx.seq_rows,
@@ -101,6 +126,9 @@ def paged_attention(ctx, out, q, k_pool, v_pool, table, num_heads: int, scale: f
     use_mma = bf16 and ctx.all_decode and ops.attention_mma_supports(num_heads, Hkv, D, page_size, True)
     if use_mma:
         NP = decode_partitions(ctx, Hkv, ops.attention_decode_mma_blocks_per_sm(D), 128)
+        if ctx.share_keys and ops.attention_balanced_supports(num_heads, Hkv, D, page_size, ctx.num_seqs):
+            balanced_attention(ctx, out, q, k_pool, v_pool, table, num_heads, scale, window)
+            return
     else:
         # SIMT: a partition is ceil(pages of the row / NP) pages, so a fixed NP cuts a row by its own length alone
         keys_per_part = 4 * page_size if fixed is None else fixed
@@ -166,6 +194,31 @@ class GQAAttention(Part):
     def streamed_weights(self):
         """The weight matrices in the order in which forward() reads them."""
         return [self.qkv.weight, self.o.weight]
+
+    def prefers_shares(self, lengths: Sequence[int], num_sms: int) -> bool:
+        """Whether a decode step over rows of so many keys should deal them in equal shares (attention_balanced.cu)
+        rather than cut every row into the same number of partitions.
+
+        In tiles of 64 keys, a block of the split-key kernel takes ceil(longest / partitions) and one of the other T / W;
+        a row that two shares cut costs both a merge through memory, and the launch about 5 us.  Measured (us, 32 query and
+        8 KV heads of 128, split-key / shares; in brackets the tiles that a split-key block has more): 16 rows of 4,000
+        keys (4) 45 / 50, 32 of 2,048 (4) 43 / 50, 18 of 125 to 2,000 (8) 23 / 22, 10 of 250 to 4,000 (8) 27 / 22, 24 of
+        2,048 (12) 42 / 40, 12 of 250 to 4,000 (15) 39 / 25, 19 of 2,000 (16) 39 / 34: from 8 tiles on.  More rows than shares
+        are no partitions but whole rows in a second round of blocks: 64 rows of 512 keys 28 / 31, 48 of 1,000 46 / 40, 64 of
+        2,048 87 / 89, 64 of 128 to 2,048 65 / 59, 64 of 256 to 4,096 124 / 96: from 16 tiles in the longest row on."""
+        N = len(lengths)
+        if N < 5 or paged_partition() is not None:          # few rows are cut into many partitions each: even anyway
+            return False
+        per_sm = ops.attention_decode_mma_blocks_per_sm(self.D)
+        parts = max(1, min((num_sms * per_sm) // max(1, self.Hkv * N), 16))
+        shares = ops.attention_balanced_shares(self.Hq, self.Hkv, self.D, N, num_sms)
+        if self.window:
+            lengths = [min(n, self.window) for n in lengths]
+        longest = -(-max(lengths) // 64)
+        if N > shares:
+            return longest >= 16
+        total = sum(lengths) / 64 + N / 2
+        return -(-longest // parts) - total / shares >= 8
 
     def forward(self, ctx, x: torch.Tensor, cache) -> Branch:
         N = x.shape[0]
