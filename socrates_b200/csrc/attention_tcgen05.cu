@@ -13,8 +13,7 @@
 //                      shared memory, MN-major (keys are the K dimension); O stays in TMEM.
 // The weights of tile i are written over the scores of tile i (same TMEM columns), there
 // are two such S/P buffers.  Three more warps only issue work: one the score products, one the
-// P.V products (a thread issues a product about every 80 ns whatever its size, so the two
-// chains have a thread each), one the TMA copies (one box per lane).  QK(i+1) goes out before
+// P.V products (the two chains wait on different barriers), one the TMA copies (one box per lane).  QK(i+1) goes out before
 // the softmax warps have finished tile i and PV(i) as soon as they have, so the tensor core
 // works on tile i+1's scores and tile i-1's product during tile i's softmax.
 // O is rescaled lazily: the exponent's reference maximum of a row only moves when the row
@@ -181,6 +180,22 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// The issuing warps walk their loops whole and one elected lane executes the products and commits (see tcgen05_gemm.cuh:
+// inside a branch of one lane every operand of a product is moved to uniform registers first, about 80 ns a product).
+// elect.sync picks the same lane each time, as commits need it to be.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(one));
+    return one != 0;
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity));
+}
+
 // four softmax warps, the warp that issues the score products, the copy-issuing warp, the warp
 // that issues the P.V products
 constexpr int THREADS = ROWS + 96;
@@ -211,7 +226,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_k, const __g
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
 
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);     // known to be uniform
     const bool issuer = warp == 4;                          // S = Q K^T
     const bool copier = warp == 5;
     const bool pv_issuer = warp == 6;                       // O += P V
@@ -347,58 +362,64 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_k, const __g
         }
     } else if (issuer) {
         // =============================================================== the warp that issues Q K^T
-        // One thread issues a tcgen05.mma about every 80 ns whatever its size (measured), and a
-        // key tile needs 8 products for the scores and 8 for P.V: issued by one thread they, not
-        // the tensor core, set the pace.  So scores and P.V have an issuing thread each; they
-        // write different accumulators and meet only through barriers.
-        if (active && (tid & 31) == 0) {
+        // Scores and P.V have an issuing warp each: each chain waits for its own barriers, and they write different
+        // accumulators.
+        const int tiles_here = __shfl_sync(0xffffffffu, n_tiles, 0);
+        if (active) {
             constexpr uint32_t idesc_qk = make_idesc(KTILE, false);
             const uint64_t dq = desc_kmajor(q_s), dk = desc_kmajor(k_s);
-            for (int i = 0; i < n_tiles; ++i) {
+            const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
+            for (int i = 0; i < tiles_here; ++i) {
                 const int b = i & 1;
-                if (!mbar_wait(smem_u32(&k_full[b]), (i >> 1) & 1)) { atomicExch(status, 11); atomicExch(&abort_flag, 1); break; }
+                if (!mbar_wait_warp(smem_u32(&k_full[b]), (i >> 1) & 1)) { atomicExch(status, 11); atomicExch(&abort_flag, 1); break; }
                 // S[b] still holds P(i-2), the A operand of PV(i-2).  The tensor core orders
                 // products by their accumulators only, not by an operand read from tensor memory,
                 // so PV(i-2) must have COMPLETED before its weights are overwritten.  v_free[b]
                 // completes once per product on buffer b, and the next one cannot come before the
                 // scores issued here: the wait is never two phases behind.
-                if (i >= 2 && !mbar_wait(smem_u32(&v_free[b]), ((i - 2) >> 1) & 1)) {
+                if (i >= 2 && !mbar_wait_warp(smem_u32(&v_free[b]), ((i - 2) >> 1) & 1)) {
                     atomicExch(status, 13); atomicExch(&abort_flag, 1); break;
                 }
-                if (*((volatile int*)&abort_flag)) break;
+                if (__any_sync(0xffffffffu, *((volatile int*)&abort_flag))) break;
                 tc_fence_after();
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < D / 16; ++kk) {
-                    // the start address sits in the low bits of a descriptor in units of 16 bytes
-                    const uint32_t pq = ((kk >> 2) * PANEL_Q + (kk & 3) * 32) >> 4;
-                    const uint32_t pk = (b * kv_bytes<D>() + (kk >> 2) * PANEL_KV + (kk & 3) * 32) >> 4;
-                    mma_ss(tmem + COL_SP + 64 * b, dq + pq, dk + pk, idesc_qk, kk > 0 ? 1u : 0u);
+                    for (int kk = 0; kk < D / 16; ++kk) {
+                        // the start address sits in the low bits of a descriptor in units of 16 bytes
+                        const uint32_t pq = ((kk >> 2) * PANEL_Q + (kk & 3) * 32) >> 4;
+                        const uint32_t pk = (b * kv_bytes<D>() + (kk >> 2) * PANEL_KV + (kk & 3) * 32) >> 4;
+                        mma_ss(tmem_u + COL_SP + 64 * b, dq + pq, dk + pk, idesc_qk, kk > 0 ? 1u : 0u);
+                    }
+                    tc_commit(smem_u32(&s_full[b]));
                 }
-                tc_commit(smem_u32(&s_full[b]));
             }
         }
     } else if (pv_issuer) {
         // =============================================================== the warp that issues P V
-        if (active && (tid & 31) == 0) {
+        const int tiles_here = __shfl_sync(0xffffffffu, n_tiles, 0);
+        if (active) {
             constexpr uint32_t idesc_pv = make_idesc(D, true);
             const uint64_t dv = desc_mnmajor(v_s, PANEL_KV >> 4);
-            for (int i = 0; i < n_tiles; ++i) {
+            const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
+            for (int i = 0; i < tiles_here; ++i) {
                 const int b = i & 1;
                 // the softmax warps have written P(i) (and zeroed unseen V rows); V(i) has landed
-                if (!mbar_wait(smem_u32(&p_ready[b]), (i >> 1) & 1)) { atomicExch(status, 16); atomicExch(&abort_flag, 1); break; }
-                if (!mbar_wait(smem_u32(&v_full[b]), (i >> 1) & 1)) { atomicExch(status, 14); atomicExch(&abort_flag, 1); break; }
-                if (*((volatile int*)&abort_flag)) break;
+                if (!mbar_wait_warp(smem_u32(&p_ready[b]), (i >> 1) & 1)) { atomicExch(status, 16); atomicExch(&abort_flag, 1); break; }
+                if (!mbar_wait_warp(smem_u32(&v_full[b]), (i >> 1) & 1)) { atomicExch(status, 14); atomicExch(&abort_flag, 1); break; }
+                if (__any_sync(0xffffffffu, *((volatile int*)&abort_flag))) break;
                 tc_fence_after();
-                const uint32_t pbase = tmem + COL_SP + 64 * b;
+                if (elect_one()) {
+                    const uint32_t pbase = tmem_u + COL_SP + 64 * b;
 #pragma unroll
-                for (int j = 0; j < KTILE / 16; ++j)
-                    mma_ts(tmem + COL_O, pbase + j * 8, dv + ((b * kv_bytes<D>() + j * 2048) >> 4), idesc_pv,
-                           (i > 0 || j > 0) ? 1u : 0u);
+                    for (int j = 0; j < KTILE / 16; ++j)
+                        mma_ts(tmem_u + COL_O, pbase + j * 8, dv + ((b * kv_bytes<D>() + j * 2048) >> 4), idesc_pv,
+                               (i > 0 || j > 0) ? 1u : 0u);
 #pragma unroll
-                for (int j = 0; j < KTILE / 16; ++j)
-                    mma_ts(tmem + COL_O, pbase + 32 + j * 8, dv + ((b * kv_bytes<D>() + j * 2048) >> 4), idesc_pv, 1u);
-                tc_commit(smem_u32(&pv_full));
-                tc_commit(smem_u32(&v_free[b]));            // V buffer b and S/P buffer b may be reused
+                    for (int j = 0; j < KTILE / 16; ++j)
+                        mma_ts(tmem_u + COL_O, pbase + 32 + j * 8, dv + ((b * kv_bytes<D>() + j * 2048) >> 4), idesc_pv, 1u);
+                    tc_commit(smem_u32(&pv_full));
+                    tc_commit(smem_u32(&v_free[b]));        // V buffer b and S/P buffer b may be reused
+                }
             }
         }
     } else if (active) {

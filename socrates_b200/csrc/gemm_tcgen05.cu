@@ -137,7 +137,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t tiles = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const int a0 = blockIdx.x * BM, b0 = blockIdx.y * BN;
     const int kb_total = (K + BK - 1) / BK;
@@ -225,7 +225,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
                 l2_prefetch(next_w + off, (uint32_t)(left < kL2Chunk ? left : kL2Chunk));
             }
         }
-    } else if (warp >= 1 && warp <= issuers && lane == 0) {
+    } else if (warp >= 1 && warp <= issuers) {
         // ---------------- MMA issuer q of `issuers`: the K blocks of its stages into accumulator q
         constexpr uint32_t idesc = make_idesc(BN);
         const int q = warp - 1;
@@ -238,7 +238,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
             if (++owner == issuers) owner = 0;
             if (++s == STAGES) { s = 0; owner = 0; parity ^= (i > 0); }
             if (owner != q) continue;
-            if (!mbar_wait(smem_u32(&full_bar[s]), parity)) {
+            if (!mbar_wait_warp(smem_u32(&full_bar[s]), parity)) {
                 atomicExch(status, 2);
                 atomicExch(&abort_flag, 1);
                 ok = false;
@@ -246,17 +246,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
             }
             tcgen05_fence_after();
             const uint32_t sa = tiles + s * stage_bytes<BN>();
-            const uint32_t sb = sa + BM * BK * 2;
+            const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + BM * BK * 2);
+            if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < BK / UMMA_K; ++k) {
-                const uint64_t da = make_smem_desc(sa + k * UMMA_K * 2);
-                const uint64_t db = make_smem_desc(sb + k * UMMA_K * 2);
-                tcgen05_mma_bf16(acc, da, db, idesc, (!first || k > 0) ? 1u : 0u);
+                for (int k = 0; k < BK / UMMA_K; ++k)      // the address is the low bits of a descriptor, in 16 bytes
+                    tcgen05_mma_bf16(acc, da + k * (UMMA_K * 2 / 16), db + k * (UMMA_K * 2 / 16), idesc,
+                                     (!first || k > 0) ? 1u : 0u);
+                tcgen05_commit(smem_u32(&empty_bar[s]));   // frees the stage when these MMAs have read it
             }
             first = false;
-            tcgen05_commit(smem_u32(&empty_bar[s]));   // frees the stage when these MMAs have read it
         }
-        tcgen05_commit(smem_u32(&accum_bar));          // arrives when every MMA of this thread has completed
+        if (elect_one()) tcgen05_commit(smem_u32(&accum_bar));     // arrives when every MMA of this thread has completed
     }
     __syncwarp();
 

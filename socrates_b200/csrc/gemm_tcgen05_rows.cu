@@ -43,7 +43,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const 
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t tiles = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const int kb_total = (K + BK - 1) / BK;
     const int n_tiles = tiles_m * tiles_n;
@@ -119,7 +119,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const 
             for (uint32_t i = it > STAGES ? it - STAGES : 0; i < it; ++i)
                 mbar_wait(smem_u32(&full_bar[i % STAGES]), (i / STAGES) & 1);
         }
-    } else if ((warp == 1 || warp == 6) && lane == 0) {
+    } else if (warp == 1 || warp == 6) {
         // ---------------- MMA issuer q (warp 1, and warp 6 when there are two)
         constexpr uint32_t idesc = make_idesc(BN);
         constexpr int NACC = acc_buffers<BN, ISSUERS>();
@@ -131,23 +131,25 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const 
         for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++j) {
             const int acc = j % NACC;
             // the epilogue must have drained this accumulator (first use of each passes at once)
-            if (j >= NACC && !mbar_wait(smem_u32(&acc_empty[acc]), ((j / NACC) - 1) & 1)) { ok = false; break; }
+            if (j >= NACC && !mbar_wait_warp(smem_u32(&acc_empty[acc]), ((j / NACC) - 1) & 1)) { ok = false; break; }
             tcgen05_fence_after();
             const uint32_t d = tmem_d + acc * ACC_STRIDE + q * BN;
             for (int i = 0; i < kb_total; ++i, ++it) {
                 const int s = it % STAGES;
-                if (!mbar_wait(smem_u32(&full_bar[s]), (it / STAGES) & 1)) { ok = false; break; }
+                if (!mbar_wait_warp(smem_u32(&full_bar[s]), (it / STAGES) & 1)) { ok = false; break; }
                 tcgen05_fence_after();
-                const uint32_t sa = tiles + s * stage_bytes<BN>();
-                const uint32_t sb_ = sa + BM * BK * 2;
+                const uint32_t sa = tiles + s * stage_bytes<BN>() + q * KPER * UMMA_K * 2;
+                const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + BM * BK * 2);
+                if (elect_one()) {
 #pragma unroll
-                for (int k = q * KPER; k < (q + 1) * KPER; ++k)
-                    tcgen05_mma_bf16(d, make_smem_desc(sa + k * UMMA_K * 2), make_smem_desc(sb_ + k * UMMA_K * 2),
-                                     idesc, (i > 0 || k > q * KPER) ? 1u : 0u);
-                tcgen05_commit(smem_u32(&empty_bar[s]));
+                    for (int k = 0; k < KPER; ++k)          // the address is the low bits of a descriptor, in 16 bytes
+                        tcgen05_mma_bf16(d, da + k * (UMMA_K * 2 / 16), db + k * (UMMA_K * 2 / 16), idesc,
+                                         (i > 0 || k > 0) ? 1u : 0u);
+                    tcgen05_commit(smem_u32(&empty_bar[s]));
+                }
             }
             if (!ok) break;
-            tcgen05_commit(smem_u32(&acc_full[acc]));
+            if (elect_one()) tcgen05_commit(smem_u32(&acc_full[acc]));
         }
         if (!ok) {
             atomicExch(status, 2);
@@ -295,7 +297,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const uint32_t tiles = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -383,7 +385,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
                 while (global_timer_ns() - t0 < 1000000ull) {}
             }
         }
-    } else if (warp == 1 && lane == 0 && rank == 0) {
+    } else if (warp == 1 && rank == 0) {
         // ---------------- MMA issuer: one thread of block 0 for the pair
         constexpr uint32_t idesc = make_idesc_pair(BN);
         uint32_t it = 0;
@@ -391,23 +393,25 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
         bool ok = true;
         for (int t = pair; t < n_tiles && ok; t += n_pairs, ++j) {
             const int acc = j & 1;
-            if (j >= 2 && !mbar_wait_cluster(smem_u32(&acc_empty[acc]), ((j >> 1) - 1) & 1)) { ok = false; break; }
+            if (j >= 2 && !__all_sync(0xffffffffu, mbar_wait_cluster(smem_u32(&acc_empty[acc]), ((j >> 1) - 1) & 1))) { ok = false; break; }
             tcgen05_fence_after();
             const uint32_t d = tmem_d + acc * ACC_COLS;
             for (int i = 0; i < kb_total; ++i, ++it) {
                 const int s = it % STAGES;
-                if (!mbar_wait(smem_u32(&full_bar[s]), (it / STAGES) & 1)) { ok = false; break; }
+                if (!mbar_wait_warp(smem_u32(&full_bar[s]), (it / STAGES) & 1)) { ok = false; break; }
                 tcgen05_fence_after();
                 const uint32_t sa = tiles + s * SB;
-                const uint32_t sb_ = sa + BM * BK * 2;
+                const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + BM * BK * 2);
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < BK / UMMA_K; ++k)
-                    tcgen05_mma_bf16_pair(d, make_smem_desc(sa + k * UMMA_K * 2), make_smem_desc(sb_ + k * UMMA_K * 2),
-                                          idesc, (i > 0 || k > 0) ? 1u : 0u);
-                tcgen05_commit_pair(smem_u32(&empty_bar[s]));        // frees the stage in both blocks
+                    for (int k = 0; k < BK / UMMA_K; ++k)
+                        tcgen05_mma_bf16_pair(d, da + k * (UMMA_K * 2 / 16), db + k * (UMMA_K * 2 / 16), idesc,
+                                              (i > 0 || k > 0) ? 1u : 0u);
+                    tcgen05_commit_pair(smem_u32(&empty_bar[s]));    // frees the stage in both blocks
+                }
             }
             if (!ok) break;
-            tcgen05_commit_pair(smem_u32(&acc_full[acc]));           // both blocks' epilogues may read
+            if (elect_one()) tcgen05_commit_pair(smem_u32(&acc_full[acc]));     // both blocks' epilogues may read
         }
         if (!ok) {
             atomicExch(status, 2);
@@ -514,7 +518,7 @@ gemm_tcgen05_pair_shares_kernel(const __grid_constant__ CUtensorMap tma_a, const
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const uint32_t tiles = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -598,7 +602,7 @@ gemm_tcgen05_pair_shares_kernel(const __grid_constant__ CUtensorMap tma_a, const
                 while (global_timer_ns() - t0 < 1000000ull) {}
             }
         }
-    } else if (warp == 1 && lane == 0 && rank == 0) {
+    } else if (warp == 1 && rank == 0) {
         // ---------------- MMA issuer: one thread of block 0 for the pair
         constexpr uint32_t idesc = make_idesc_pair(BN);
         uint32_t it = 0;
@@ -608,23 +612,25 @@ gemm_tcgen05_pair_shares_kernel(const __grid_constant__ CUtensorMap tma_a, const
         Piece pc;
         for (; ok && walk.next(pc); ++j) {
             const int acc = j & 1;
-            if (j >= 2 && !mbar_wait_cluster(smem_u32(&acc_empty[acc]), ((j >> 1) - 1) & 1)) { ok = false; break; }
+            if (j >= 2 && !__all_sync(0xffffffffu, mbar_wait_cluster(smem_u32(&acc_empty[acc]), ((j >> 1) - 1) & 1))) { ok = false; break; }
             tcgen05_fence_after();
             const uint32_t d = tmem_d + acc * ACC_COLS;
             for (int i = pc.kb0; i < pc.kb1; ++i, ++it) {
                 const int s = it % STAGES;
-                if (!mbar_wait(smem_u32(&full_bar[s]), (it / STAGES) & 1)) { ok = false; break; }
+                if (!mbar_wait_warp(smem_u32(&full_bar[s]), (it / STAGES) & 1)) { ok = false; break; }
                 tcgen05_fence_after();
                 const uint32_t sa = tiles + s * SB;
-                const uint32_t sb_ = sa + BM * BK * 2;
+                const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + BM * BK * 2);
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < BK / UMMA_K; ++k)
-                    tcgen05_mma_bf16_pair(d, make_smem_desc(sa + k * UMMA_K * 2), make_smem_desc(sb_ + k * UMMA_K * 2),
-                                          idesc, (i > pc.kb0 || k > 0) ? 1u : 0u);
-                tcgen05_commit_pair(smem_u32(&empty_bar[s]));        // frees the stage in both blocks
+                    for (int k = 0; k < BK / UMMA_K; ++k)
+                        tcgen05_mma_bf16_pair(d, da + k * (UMMA_K * 2 / 16), db + k * (UMMA_K * 2 / 16), idesc,
+                                              (i > pc.kb0 || k > 0) ? 1u : 0u);
+                    tcgen05_commit_pair(smem_u32(&empty_bar[s]));    // frees the stage in both blocks
+                }
             }
             if (!ok) break;
-            tcgen05_commit_pair(smem_u32(&acc_full[acc]));           // both blocks' epilogues may read
+            if (elect_one()) tcgen05_commit_pair(smem_u32(&acc_full[acc]));     // both blocks' epilogues may read
         }
         if (!ok) {
             atomicExch(status, 2);
