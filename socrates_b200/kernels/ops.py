@@ -531,14 +531,15 @@ def attention_prefill_tcgen05(out: torch.Tensor, q: torch.Tensor, k_pool: torch.
                               sink: Optional[float] = None, keep_first: int = 0,
                               out_float: Optional[torch.Tensor] = None, softcap: float = 0.0,
                               slopes: Optional[torch.Tensor] = None, chunk: int = 0,
-                              skip_single: bool = False) -> None:
+                              skip_single: bool = False, dist_bias: Optional[torch.Tensor] = None) -> None:
     """Paged causal attention of prompt portions on tcgen05 (scores and P.V in tensor
     memory, pages brought in by TMA).  Arguments as `attention_prefill_mma`, plus the int32
     status word that receives a non-zero code if a bounded wait inside the kernel gave up.
     `keep_first`: a window also sees the first so many keys of its row.  `out_float` (float32
     [N, Hq*D]): the rows go there unrounded instead of to `out` (which may then be None).
     `softcap`, `slopes`, `chunk` as in `attention_decode_mma`.  `skip_single`: requests that bring one
-    token are left out (see `attention_decode_balanced`); their rows of `out` are not written."""
+    token are left out (see `attention_decode_balanced`); their rows of `out` are not written.  `dist_bias`
+    float32 [Hq, L]: joins the score of the key at distance min(d, L - 1), after the cap."""
     N = q.shape[0]
     pages, Hkv, BS, D = k_pool.shape
     R = seq_rows.numel()
@@ -556,6 +557,12 @@ def attention_prefill_tcgen05(out: torch.Tensor, q: torch.Tensor, k_pool: torch.
     _want(seq_rows, "seq_rows", torch.int32, (R,))
     _want(seq_first_pos, "seq_first_pos", torch.int32, (R,))
     _want(status, "status", torch.int32)
+    L = 0
+    if dist_bias is not None:
+        _want(dist_bias, "dist_bias", torch.float32)
+        if dist_bias.dim() != 2 or dist_bias.shape[0] != num_heads:
+            raise KernelError(f"dist_bias must be [{num_heads}, L], got {tuple(dist_bias.shape)}")
+        L = dist_bias.shape[1]
     # optional: out *= sigmoid(gate) (gate [N, >= Hq] or, with gate_per_dim, [N, >= Hq*D], bfloat16) and a sink,
     # a score whose exponential joins the softmax denominator without a value
     gate_stride = _gate_stride(gate, q, N, num_heads * D if gate_per_dim else num_heads)
@@ -565,7 +572,7 @@ def attention_prefill_tcgen05(out: torch.Tensor, q: torch.Tensor, k_pool: torch.
         _ptr(seq_starts), _ptr(seq_rows), _ptr(seq_first_pos), R, N, num_heads, Hkv, D, BS, int(window),
         float(scale), _ptr(status), _ptr(gate), gate_stride, int(gate_per_dim), int(sink is not None),
         float(sink or 0.0), int(keep_first), _ptr(out_float), float(softcap), _slopes(slopes, num_heads), int(chunk),
-        int(skip_single), _stream()), "attention_prefill_tcgen05")
+        int(skip_single), _ptr(dist_bias), L, _stream()), "attention_prefill_tcgen05")
 
 
 # ---------------------------------------------------------------------------------------------

@@ -124,8 +124,14 @@ class WindowBiasAttention(Part):
             ops.short_conv_tail(tail, qkvg, self.in_bias, self.taps, ctx.seq_starts, ctx.seq_rows)
         attn = ctx.buffers.take("wa_attn", N, (self.H * self.dv,), ctx.dtype)
         gate = qkvg[:, self.C:self.C + self.H]
-        if (not ctx.all_decode and N >= 4 * ctx.num_seqs
-                and ops.attention_bias_tile_supports(self.H, self.G, self.dk, self.dv, ctx.dtype)):
+        portions = not ctx.all_decode and N >= 4 * ctx.num_seqs
+        if (portions and ctx.dtype == torch.bfloat16 and self.dk == self.dv and ctx.status is not None
+                and ops.attention_tcgen05_supports(self.H, self.G, self.dk, k_pool.shape[2])):
+            ops.attention_prefill_tcgen05(attn, q, k_pool, v_pool, table, ctx.seq_starts, ctx.seq_rows, ctx.seq_first_pos,
+                                          self.H, self.scale, ctx.status, self.window or 0, gate=gate,
+                                          softcap=self.softcap, dist_bias=self.dist_bias)
+            return Branch(self.o(ctx, attn, self.out_buffer, out="partial"))
+        if (portions and ops.attention_bias_tile_supports(self.H, self.G, self.dk, self.dv, ctx.dtype)):
             # prompt portions: a tile of a request's consecutive tokens per block shares the keys it reads
             ops.attention_bias_tile(attn, q, k_pool, v_pool, table, ctx.seq_starts, ctx.seq_rows, ctx.seq_first_pos,
                                     self.H, self.scale, self.window or 0, self.softcap, self.dist_bias, gate=gate)
