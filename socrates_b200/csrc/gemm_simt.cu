@@ -1,12 +1,17 @@
 // C[M,N] = A[M,K] * W[N,K]^T on the CUDA cores, float32 FMA accumulation.
 //
-// This is the matrix product of the true 32-bit path (no tensor-core kind, no TF32)
-// and the fallback of the bfloat16 path for shapes the tensor-core kernel refuses.
+// This is the fallback of the bfloat16 path for shapes the tensor-core kernel refuses and of the true 32-bit
+// path (no tensor-core kind, no TF32) for what gemm_f32.cu does not take (K % 4 != 0, a cut product).
 // Any M, N, K; A, W and C each float32 or bfloat16.  With splits > 1 the K range is
 // cut into `splits` parts and part z writes float32 partial sums to C + z*M*N.
 #include "common.cuh"
 
 using namespace sb;
+
+namespace sb {                          // gemm_f32.cu
+bool gemm_f32_takes(const void* C, const void* A, const void* W, int M, int N, int K);
+int gemm_f32(float* C, const float* A, const float* W, int M, int N, int K, cudaStream_t stream);
+}
 
 namespace {
 
@@ -86,6 +91,11 @@ extern "C" int sb_gemm_simt(void* C, const void* A, const void* W, int M, int N,
     SB_REQUIRE(splits == 1 || c_dtype == SB_F32, "gemm_simt: partial sums of a split product are float32");
     SB_REQUIRE((M + BM - 1) / BM <= 65535, "gemm_simt: M=%d is too large", M);
     if (M == 0) return 0;
+    if (a_dtype == SB_F32 && w_dtype == SB_F32 && c_dtype == SB_F32 && splits == 1 && sb::gemm_f32_takes(C, A, W, M, N, K)) {
+        const int rc = sb::gemm_f32((float*)C, (const float*)A, (const float*)W, M, N, K, stream);
+        if (rc != 0) return rc;
+        SB_LAUNCH_CHECK();
+    }
     const int key = a_dtype * 4 + w_dtype * 2 + c_dtype;
     typedef __nv_bfloat16 bf;
     switch (key) {
