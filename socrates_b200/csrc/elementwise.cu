@@ -211,12 +211,14 @@ extern "C" int sb_add_rmsnorm(float* residual, const float* delta, int S, long l
     const bool vec = d % 4 == 0 && delta_stride % 4 == 0 &&
                      ((reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(delta) |
                        reinterpret_cast<uintptr_t>(gain) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-    // vector kernel: one float4 column per thread where the row allows it (few rows are the
-    // decode regime, where the S partial sums of a column should all be in flight at once)
+    // vector kernel: one float4 column per thread where the row allows it (few rows are the decode
+    // regime, where the S partial sums of a column should all be in flight at once; so are 65 to 256
+    // rows behind a product in many parts)
+    const bool deep = M <= 64 || (M <= 256 && S > 2);
     int threads = d >= 2048 ? 512 : 256;
     if (vec) {
         threads = ((d / 4 + 31) / 32) * 32;
-        if (threads > (M <= 64 ? 640 : 768)) threads = M <= 64 ? 640 : 768;
+        if (threads > (deep ? 640 : 768)) threads = deep ? 640 : 768;
         if (M > 512 && threads > 256) threads = 256;
     }
 #define SB_NORM_LAUNCH(KERNEL, ...)                                                                      \
@@ -227,11 +229,11 @@ extern "C" int sb_add_rmsnorm(float* residual, const float* delta, int S, long l
                    (decltype(sb_out_type<__VA_ARGS__>()))out, row_index, d, eps, write_residual);        \
     } while (0)
     if (dtype == SB_F32) {
-        if (vec && M <= 64) SB_NORM_LAUNCH(add_rmsnorm_vec_kernel, float, 16);
+        if (vec && deep) SB_NORM_LAUNCH(add_rmsnorm_vec_kernel, float, 16);
         else if (vec) SB_NORM_LAUNCH(add_rmsnorm_vec_kernel, float, 2);
         else SB_NORM_LAUNCH(add_rmsnorm_kernel, float);
     } else if (dtype == SB_BF16) {
-        if (vec && M <= 64) SB_NORM_LAUNCH(add_rmsnorm_vec_kernel, __nv_bfloat16, 16);
+        if (vec && deep) SB_NORM_LAUNCH(add_rmsnorm_vec_kernel, __nv_bfloat16, 16);
         else if (vec) SB_NORM_LAUNCH(add_rmsnorm_vec_kernel, __nv_bfloat16, 2);
         else SB_NORM_LAUNCH(add_rmsnorm_kernel, __nv_bfloat16);
     } else {
@@ -610,8 +612,40 @@ __global__ void qk_norm_rope_kvwrite_rows_kernel(
         const int page = block_table[(size_t)token_rows[n] * table_width + pos / BS];
         kv_slot = ((size_t)page * Hkv * BS + (pos % BS)) * D;            // + kh * BS * D per KV head
     }
+    // A lane keeps its cosines and sines (the sign of its half folded in): they are the same for every head.  With the next
+    // head's elements on their way as well, 2,048 tokens of 48 heads: 23 -> 20 us.
+    const bool turns = R == D;
+    float c_own[EXTRA ? 1 : VPL], s_own[EXTRA ? 1 : VPL];
+    if constexpr (!EXTRA) {
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) {
+            c_own[i] = turns ? cs[(l & 7) * VPL + i] : 1.f;
+            s_own[i] = turns ? (l < 8 ? -sn[l * VPL + i] : sn[(l & 7) * VPL + i]) : 0.f;
+        }
+    }
     const int head_end = min(n_heads, (int)(blockIdx.y + 1) * heads_per_block);
     const int nwarps = blockDim.x >> 5;
+    // the next head's elements are on their way while one is worked on
+    auto fetch = [&](int head, float (&v)[VPL]) {
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) v[i] = 0.f;
+        if (head < head_end && (head < Hq || write_kv)) {
+            const size_t base = ((size_t)n * n_heads + head) * D + l * VPL;
+            if (parts != nullptr) {
+                for (int s = 0; s < S; ++s) {               // added in the order s = 0, 1, ...
+                    const Pack<float, VPL> p = *reinterpret_cast<const Pack<float, VPL>*>(parts + s * part_stride + base);
+#pragma unroll
+                    for (int i = 0; i < VPL; ++i) v[i] += p.v[i];
+                }
+            } else {
+                const Pack<T, VPL> p = *reinterpret_cast<const Pack<T, VPL>*>(qkv + base);
+#pragma unroll
+                for (int i = 0; i < VPL; ++i) v[i] = to_float(p.v[i]);
+            }
+        }
+    };
+    float ahead[VPL];
+    fetch(blockIdx.y * heads_per_block + 2 * warp + sub, ahead);
     for (int head0 = blockIdx.y * heads_per_block + 2 * warp; head0 < head_end; head0 += 2 * nwarps) {
         const int head = head0 + sub;
         const bool is_q = head < Hq;
@@ -620,21 +654,8 @@ __global__ void qk_norm_rope_kvwrite_rows_kernel(
         const bool live = head < head_end && (is_q || write_kv);
         float y[VPL];
 #pragma unroll
-        for (int i = 0; i < VPL; ++i) y[i] = 0.f;
-        if (live) {
-            const size_t base = ((size_t)n * n_heads + head) * D + l * VPL;
-            if (parts != nullptr) {
-                for (int s = 0; s < S; ++s) {               // added in the order s = 0, 1, ...
-                    const Pack<float, VPL> p = *reinterpret_cast<const Pack<float, VPL>*>(parts + s * part_stride + base);
-#pragma unroll
-                    for (int i = 0; i < VPL; ++i) y[i] += p.v[i];
-                }
-            } else {
-                const Pack<T, VPL> p = *reinterpret_cast<const Pack<T, VPL>*>(qkv + base);
-#pragma unroll
-                for (int i = 0; i < VPL; ++i) y[i] = to_float(p.v[i]);
-            }
-        }
+        for (int i = 0; i < VPL; ++i) y[i] = ahead[i];
+        fetch(head + 2 * nwarps, ahead);
         if (EXTRA && live && extra.bias != nullptr) {
             const float* b = extra.bias + (size_t)head * D + l * VPL;
 #pragma unroll
@@ -675,13 +696,13 @@ __global__ void qk_norm_rope_kvwrite_rows_kernel(
                 o.v[i] = from_float<T>(r);
             }
         }
-        const bool rotate = !is_v && R == D;
+        if constexpr (!EXTRA) {
+            const bool rotate = !is_v && turns;
 #pragma unroll
-        for (int i = 0; i < VPL && !EXTRA; ++i) {
-            const float partner = __shfl_xor_sync(0xffffffffu, y[i], 8);
-            const float c = cs[(l & 7) * VPL + i], s = sn[(l & 7) * VPL + i];
-            const float r = l < 8 ? y[i] * c - partner * s : y[i] * c + partner * s;
-            o.v[i] = from_float<T>(rotate ? r : y[i]);
+            for (int i = 0; i < VPL; ++i) {
+                const float partner = __shfl_xor_sync(0xffffffffu, y[i], 8);
+                o.v[i] = from_float<T>(rotate ? y[i] * c_own[i] + partner * s_own[i] : y[i]);
+            }
         }
         if (!live) continue;
         T* dst;
