@@ -112,16 +112,16 @@ namespace {
 // SWAP = false: lanes are rows of C (m), columns are columns of C (n).
 // SWAP = true : lanes are columns of C (n), columns are rows of C (m).
 //
-// A thread issues a tcgen05.mma about every 80 ns however narrow the tile, which for the narrow
-// tiles of weight streaming is longer than the tile's loads take.  With SWAP, `issuers` (1 to
-// kMaxIssuers) threads therefore share the issuing, each into an accumulator of its own, and the
-// epilogue adds the accumulators.  A ring stage always belongs to the same thread (stage s to
-// thread s mod issuers): a thread that met only some of a stage's uses could not tell, from the
+// With SWAP and few columns, `issuers` (1 to kMaxIssuers) warps share the issuing of products (for the narrow
+// tiles of weight streaming one warp's waits and commits take longer than the tile's loads), each into an accumulator of its own, and the
+// epilogue adds the accumulators.  A ring stage always belongs to the same warp (stage s to
+// warp s mod issuers): a warp that met only some of a stage's uses could not tell, from the
 // parity it waits for, a stage that has been refilled from one that has not been filled yet.
 constexpr int kMaxIssuers = 3;
 constexpr int kDefaultIssuers = 2;      // measured: 2.58 ms a decode step against 2.62 (one) and 2.59 (three)
+template <int BN, bool SWAP> constexpr int max_issuers() { return SWAP && BN <= 64 ? kMaxIssuers : 1; }
 template <int BN, bool SWAP> constexpr int acc_cols() {
-    constexpr int want = (SWAP ? kMaxIssuers : 1) * BN;
+    constexpr int want = max_issuers<BN, SWAP>() * BN;
     return want <= 32 ? 32 : want <= 64 ? 64 : want <= 128 ? 128 : want <= 256 ? 256 : 512;
 }
 
@@ -144,7 +144,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
     const int kb_begin = blockIdx.z * kb_per_split;
     const int kb_end = min(kb_total, kb_begin + kb_per_split);
     const int kb_count = kb_end - kb_begin;
-    if (!SWAP) issuers = 1;
+    if (max_issuers<BN, SWAP>() == 1) issuers = 1;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -275,7 +275,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
             uint32_t r[16];
             const uint32_t at = tmem_d + (static_cast<uint32_t>(warp * 32) << 16) + c0;
             tmem_ld16(at, r);
-            if constexpr (SWAP) {
+            if constexpr (max_issuers<BN, SWAP>() > 1) {
                 // the accumulators of the other issuing threads count where those had a K block
                 // (all are read, so that the loads overlap; what an unused one holds is dropped)
                 const int used = min(issuers, kb_count);
@@ -427,6 +427,24 @@ int dispatch(const void* A, const void* W, void* C, int M, int N, int K, int spl
         if (bn == 32) return launch<32, 5, true, TC>(ma, mb, C, M, N, K, grid, kb_per_split, status, stream);
         return launch<64, 4, true, TC>(ma, mb, C, M, N, K, grid, kb_per_split, status, stream);
     }
+    if (variant == 5) {
+        // Weight streaming for up to 256 rows (and more in passes of 256): the weights on the lanes, all rows as columns, so
+        // that a K block's weights reach one SM once; two blocks an SM up to 128 rows, one beyond.
+        const int bn = M <= 96 ? 96 : (M <= 128 ? 128 : (M <= 192 ? 192 : 256));
+        if (epi != 0) {
+            sb_set_error("gemm_tcgen05: the streaming kernel has no gated epilogue for more than 64 rows");
+            return SB_ERR_ARG;
+        }
+        if (!get_map(&ma, W, N, K, BM) || !get_map(&mb, A, M, K, bn)) {
+            sb_set_error("gemm_tcgen05: cuTensorMapEncodeTiled failed (M=%d N=%d K=%d)", M, N, K);
+            return SB_ERR_ARG;
+        }
+        dim3 grid((N + BM - 1) / BM, (M + bn - 1) / bn, splits);
+        if (bn == 96) return launch<96, 3, true, TC>(ma, mb, C, M, N, K, grid, kb_per_split, status, stream);
+        if (bn == 128) return launch<128, 3, true, TC>(ma, mb, C, M, N, K, grid, kb_per_split, status, stream);
+        if (bn == 192) return launch<192, 5, true, TC>(ma, mb, C, M, N, K, grid, kb_per_split, status, stream);
+        return launch<256, 4, true, TC>(ma, mb, C, M, N, K, grid, kb_per_split, status, stream);
+    }
     if (splits == 1 && N >= 128 && variant != 4)      // the persistent kernels (gemm_tcgen05_rows.cu)
         return sb::gemm_tcgen05_many_rows(A, W, C, M, N, K, sizeof(TC) == 2 ? SB_BF16 : SB_F32, status, variant, epi, stream);
     if (epi != 0) {
@@ -455,6 +473,7 @@ int dispatch(const void* A, const void* W, void* C, int M, int N, int K, int spl
 //          (the default there is the persistent kernel); 128, 160, 256 = that tile width
 //          in the persistent kernel instead of the one it would choose; 1128, 1160, 1192,
 //          1256 = the pair kernel (two SMs per tile, cta_group::2) with tiles 256 x (variant - 1000);
+//          5 = the weight-streaming kernel for more than 64 rows (StepContext.wide_splits says where it pays);
 //          2000 = the pair kernel dealing equal shares of K blocks, float32 partial sums
 //          [parts, M, N] with *splits_io == sb_gemm_tcgen05_shares_parts(M, N, K).
 // epilogue: 0 = C[M,N]; 1 = W interleaves gate and up rows and C is [M, N/2] = up * silu(gate); 2 = the same with

@@ -153,6 +153,9 @@ class StepContext:
             return 1
         N, K = w.shape
         if M > 64:
+            parts = self.wide_splits(M, w, x_dtype)
+            if parts:
+                return parts
             parts = self.gemm_shares(M, w, x_dtype) if shares else 0
             if parts:
                 return parts
@@ -171,6 +174,25 @@ class StepContext:
         want = max(1, (2 * self.num_sms) // tiles)
         most = max(1, (-(-K // 64)) // 2)
         return ops.gemm_tcgen05_splits(K, min(want, most, 16))
+
+    def wide_splits(self, M: int, w: torch.Tensor, x_dtype: torch.dtype) -> int:
+        """K parts of the weight-streaming kernel for 65 to 256 rows whose output is partial sums (the weights on the
+        lanes, all rows as columns of one tile: every SM reads its weights once, where tiles of 128 rows read them
+        twice and 256-wide ones leave half of the SMs idle), else 0.
+
+        As many parts as there are places (two blocks an SM up to 128 rows, one beyond), at least four K blocks each; it
+        takes three parts to beat the other kernels.  Measured (us, before / so): 187 rows: 2,560 x 4,096 16.8 / 11.4,
+        2,560 x 9,728 26.1 / 16.7, 6,144 x 2,560 16.8 / 13.3, 5,120 x 25,600 70.8 / 59.5, 4,096 x 12,288 30.5 / 28.7; 72
+        rows: 13.0 / 8.1, 21.7 / 12.9, 12.1 / 9.7, 56.0 / 54.4, 27.0 / 24.1.  256 columns are a heavier tile: there only
+        where nine tenths of the SMs get a block (2,560 x 9,728 26.5 / 19.3, but 4,096 x 12,288 31.8 / 33.8)."""
+        if not 64 < M <= 256 or not self.uses_tensor_cores(x_dtype, w):
+            return 0
+        N, K = w.shape
+        tiles = -(-N // 128)
+        parts = min((2 if M <= 128 else 1) * self.num_sms // tiles, -(-K // 64) // 4, 14)
+        if parts < 3 or (M > 192 and 10 * tiles * parts < 9 * self.num_sms):
+            return 0
+        return ops.gemm_tcgen05_splits(K, parts)
 
     def gemm_shares(self, M: int, w: torch.Tensor, x_dtype: torch.dtype) -> int:
         """Parts of the pair kernel in equal shares of K blocks if a product of M rows whose output
@@ -214,6 +236,9 @@ class StepContext:
             M = x.shape[0]
             if M > 64 and out.dim() == 3 and epilogue == 0 and S == self.gemm_shares(M, w, x.dtype) and S > 0:
                 ops.gemm_tcgen05(out, x, w, self.status, S, variant=ops.SHARES_VARIANT)
+                return
+            if S > 1 and epilogue == 0 and S == self.wide_splits(M, w, x.dtype):
+                ops.gemm_tcgen05(out, x, w, self.status, S, variant=ops.WIDE_VARIANT)
                 return
             ops.gemm_tcgen05(out if out.dim() == 3 and S > 1 else out.view(out.shape[-2], out.shape[-1]),
                              x, w, self.status, S, epilogue=epilogue, prefetch=self._next_weights(w, S))

@@ -292,6 +292,7 @@ def gemm_tcgen05_splits(K: int, splits: int) -> int:
     return library().sb_gemm_tcgen05_splits(int(K), int(splits))
 
 
+WIDE_VARIANT = 5           # gemm_tcgen05 variant: the weight-streaming kernel for more than 64 rows
 SHARES_VARIANT = 2000      # gemm_tcgen05 variant: the pair kernel dealing equal shares of K blocks
 
 

@@ -243,3 +243,31 @@ def test_gemm_tcgen05_refuses(ops):
         ops.gemm_tcgen05(torch.empty(4, 8, dtype=torch.float32, device=DEV), a, w, status)
     with pytest.raises(KernelError):
         ops.gemm_tcgen05(torch.empty(4, 8, device=DEV), a.float(), w, status)
+
+
+@pytest.mark.parametrize("M", [65, 96, 97, 128, 129, 187, 192, 193, 256])
+@pytest.mark.parametrize("N,K,S", [(2560, 4096, 7), (200, 200, 4), (128, 64, 1), (130, 1000, 3)])
+def test_weight_streaming_for_up_to_256_rows(ops, M, N, K, S):
+    """The weights on the lanes and all rows as columns: edges of the column widths, rows and columns past the end,
+    parts of unequal K."""
+    a, w, want = operands(M, N, K, seed=M)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    S = ops.gemm_tcgen05_splits(K, S)
+    out = torch.full((S, M, N), float("nan"), dtype=torch.float32, device=DEV)
+    ops.gemm_tcgen05(out, a, w, status, S, variant=ops.WIDE_VARIANT)
+    close(out.double().sum(0), want, K, False)
+    assert int(status.item()) == 0
+
+
+def test_weight_streaming_is_chosen_for_partial_sums_of_short_portions(ops):
+    from socrates_b200.engine.context import Buffers, StepContext
+    ctx = StepContext(torch.bfloat16, torch.device(DEV), Buffers(64, DEV), 1, 1, None, None, None, None, None, None,
+                      None, all_decode=False, max_context=1, num_sms=148,
+                      status=torch.zeros(1, dtype=torch.int32, device=DEV))
+    a, w, want = operands(187, 2560, 9728, seed=4)
+    S = ctx.gemm_splits(187, w, torch.bfloat16)
+    assert S == 7 and ctx.wide_splits(64, w, torch.bfloat16) == 0 and ctx.wide_splits(257, w, torch.bfloat16) == 0
+    out = torch.full((S, 187, 2560), float("nan"), dtype=torch.float32, device=DEV)
+    ctx.gemm(out, a, w)
+    close(out.double().sum(0), want, 9728, False)
+    assert int(ctx.status.item()) == 0
