@@ -31,7 +31,7 @@ COMMON_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr",
                 "-Xcompiler", "-fPIC"]
 
 # Sources of the core library, in link order.
-CORE_SOURCES = ["errors.cu", "elementwise.cu", "sampling.cu", "gemm_simt.cu", "gemm_f32.cu", "attention_simt.cu",
+CORE_SOURCES = ["errors.cu", "run_calls.cu", "elementwise.cu", "sampling.cu", "gemm_simt.cu", "gemm_f32.cu", "attention_simt.cu",
                 "gemm_tcgen05.cu", "gemm_tcgen05_rows.cu", "attention_mma.cu", "attention_decode.cu", "attention_balanced.cu",
                 "attention_tcgen05.cu", "fold_norm.cu", "short_conv.cu", "retention.cu", "selective_scan.cu",
                 "attention_bias.cu", "delta_rule.cu", "moe_route.cu", "attention_diff.cu", "hyper_norm.cu",

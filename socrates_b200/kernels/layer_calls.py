@@ -1,0 +1,109 @@
+"""The launches of a layer, recorded while it runs once and handed to the library for the layers that are like it.
+
+Within a step, layers of one shape make the same calls with the same arguments but for the addresses of their weights and
+pages.  `Recording` collects a layer's calls as the words that `sb_run_calls` takes (csrc/run_calls.cu) and finds in them
+the places that hold the layer's own addresses; `run` fills in another layer's and launches all of it in one call.  A
+recording lives for one step: nothing is kept from one step to the next, and buffers, scratch, sizes and the stream are the
+step's.
+"""
+
+from __future__ import annotations
+
+import ctypes
+import struct
+from typing import Dict, List, Optional, Sequence, Tuple
+
+import numpy as np
+import torch
+
+from .library import F, P, Counters, KernelError, _SIGNATURES, library, set_recorder
+
+# the entry points that a recorded layer may consist of, by their number in run_calls.cu
+ENTRIES = {"sb_add_rmsnorm": 0, "sb_gemm_tcgen05": 1, "sb_gemm_simt": 2, "sb_qk_norm_rope_kvwrite": 3, "sb_silu_mul": 4,
+           "sb_attention_simt": 5, "sb_attention_prefill_tcgen05": 6, "sb_attention_prefill_mma": 7,
+           "sb_attention_balanced": 8, "sb_attention_decode_mma": 9, "sb_attention_decode_stream": 10}
+# host-only questions that a layer may ask while it is recorded
+_QUESTIONS = ("_supports", "_splits", "_parts", "_shares", "_kernels", "_blocks_per_sm", "sb_last_error",
+              "sb_set_dependent_launch")
+
+
+class _Recorder:
+    """Stands in for the library: entry points run as ever and leave their name and arguments."""
+
+    def __init__(self, lib):
+        self.lib = lib
+        self.calls: List[Tuple[str, tuple]] = []
+        self.complete = True            # False once something ran that cannot be repeated from words
+
+    def __getattr__(self, name):
+        real = getattr(self.lib, name)
+        if name in ENTRIES:
+            def entry(*args):
+                self.calls.append((name, args))
+                return real(*args)
+            return entry
+        if not name.endswith(_QUESTIONS):
+            self.complete = False
+        return real
+
+
+def _word(kind, value, keep: list) -> int:
+    if kind is F:
+        return struct.unpack("<I", struct.pack("<f", value))[0]
+    if kind is P:
+        if value is None:
+            return 0
+        if not isinstance(value, int):                      # byref(c_int): a number on the host, as the call left it
+            keep.append(value._obj)
+            return ctypes.addressof(value._obj)
+    return int(value)
+
+
+class Recording:
+    """`with Recording(addresses):` runs a layer; `addresses` are the layer's own device addresses, in an order that
+    other layers' follow."""
+
+    def __init__(self, addresses: Sequence[int]):
+        self.addresses = list(addresses)
+        self.words: Optional[np.ndarray] = None
+        self._keep: list = []
+
+    def __enter__(self) -> "Recording":
+        self._recorder = _Recorder(library())
+        self._launches = Counters.launches
+        set_recorder(self._recorder)
+        return self
+
+    def __exit__(self, kind, value, trace):
+        set_recorder(None)
+        self.launches = Counters.launches - self._launches
+        if kind is not None or not self._recorder.complete or len(set(self.addresses)) != len(self.addresses):
+            return False
+        index: Dict[int, int] = {a: i for i, a in enumerate(self.addresses)}
+        words, places, which = [], [], []
+        for name, args in self._recorder.calls:
+            words.append(ENTRIES[name])
+            for t, v in zip(_SIGNATURES[name], args):
+                if t is P and isinstance(v, int) and v in index:
+                    places.append(len(words))
+                    which.append(index[v])
+                words.append(_word(t, v, self._keep))
+        self.words = np.array([w - (1 << 64) if w >= 1 << 63 else w for w in words], dtype=np.int64)
+        self._places, self._which = np.array(places, dtype=np.intp), np.array(which, dtype=np.intp)
+        self._done = ctypes.c_int(0)
+        return False
+
+    @property
+    def usable(self) -> bool:
+        return self.words is not None
+
+    def run(self, addresses: Sequence[int]) -> None:
+        """The recorded calls with another layer's addresses."""
+        words = self.words
+        words[self._places] = np.array(addresses, dtype=np.int64)[self._which]
+        lib = library()
+        rc = lib.sb_run_calls(words.ctypes.data, len(words), ctypes.byref(self._done))
+        if rc != 0:
+            raise KernelError(f"call {self._done.value} of a recorded layer: "
+                              f"{lib.sb_last_error().decode(errors='replace')} (code {rc})")
+        Counters.launches += self.launches

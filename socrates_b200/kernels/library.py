@@ -10,6 +10,7 @@ model/kernels/__init__.py:82-92 require_cuda_kernel).
 from __future__ import annotations
 
 import ctypes
+import threading
 from ctypes import c_char_p, c_float, c_int, c_longlong, c_void_p
 from typing import Optional
 
@@ -28,6 +29,8 @@ P, I, F, LL = c_void_p, c_int, c_float, c_longlong
 _SIGNATURES = {
     "sb_abi_version": [],
     "sb_set_dependent_launch": [I],
+    "sb_run_calls": [P, I, P],
+    "sb_run_calls_arity": [I],
     "sb_embed": [P, P, P, I, I, I, I, P, F, P],
     "sb_add_rmsnorm": [P, P, I, LL, P, P, P, I, I, F, I, P],
     "sb_qk_norm_rope_kvwrite": [P, P, I, LL, P, P, P, P, P, P, I, P, P, P, I, I, F, I, I, I, I, I, I, I, I, I, P, I, F, I, I, I, F, P, P],
@@ -112,9 +115,22 @@ def declare(lib: ctypes.CDLL, signatures: dict) -> None:
     lib.sb_last_error.restype = c_char_p
 
 
+class _Local(threading.local):
+    recorder = None         # stands in for the library in this thread (see layer_calls.py)
+
+
+_local = _Local()
+
+
+def set_recorder(recorder) -> None:
+    _local.recorder = recorder
+
+
 def library() -> ctypes.CDLL:
     """The loaded CUDA library; built at first call.  Raises if that is not possible."""
     global _lib, _lib_path
+    if _local.recorder is not None:
+        return _local.recorder
     if _lib is None:
         try:
             path = build_core()

@@ -195,6 +195,10 @@ class GQAAttention(Part):
         """The weight matrices in the order in which forward() reads them."""
         return [self.qkv.weight, self.o.weight]
 
+    def replay_tensors(self):
+        inv_freq, _ = self.position.tables(self.o.weight.device)
+        return [t for t in (self.qkv.weight, self.o.weight, self.q_gain, self.k_gain, inv_freq) if t is not None]
+
     def prefers_shares(self, lengths: Sequence[int], num_sms: int) -> bool:
         """Whether a decode step over rows of so many keys should deal them in equal shares (attention_balanced.cu)
         rather than cut every row into the same number of partitions.

@@ -52,6 +52,16 @@ class PreNormBlock:
         return [*getattr(self.mixer, "streamed_weights", list)(),
                 *getattr(self.feed_forward, "streamed_weights", list)()]
 
+    def replay_parts(self):
+        """The layer's parts if its kernels are given nothing of the layer's own but `replay_tensors()` (and its pages), or
+        None: another layer of the same specs then makes the same calls with its own tensors in these places
+        (kernels/layer_calls.py).  The very class of a part must say so: a subclass may launch other things."""
+        parts = self.parts()
+        return parts if all("replay_tensors" in type(p).__dict__ for p in parts) else None
+
+    def replay_tensors(self):
+        return [t for p in self.parts() for t in p.replay_tensors()]
+
     def forward(self, ctx, stream: ResidualStream, cache) -> None:
         h = self.norms[0].apply(ctx, stream)
         stream.pending = self.mixer.forward(ctx, h, cache)

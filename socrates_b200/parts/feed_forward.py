@@ -49,6 +49,9 @@ class SwiGLU(Part):
         """The weight matrices in the order in which forward() reads them."""
         return [self.gate_up.weight, self.down.weight]
 
+    def replay_tensors(self):
+        return [self.gate_up.weight, self.down.weight]
+
     def forward(self, ctx, x: torch.Tensor) -> Branch:
         N = x.shape[0]
         if ctx.can_fuse_silu_mul(N, self.gate_up.weight, x.dtype):

@@ -69,6 +69,9 @@ class RMSNorm(Part):
         g = tensors[self.tensor]
         self.gain = (g + self.offset).contiguous() if self.offset else g
 
+    def replay_tensors(self):
+        return [self.gain]
+
     def apply(self, ctx, stream: ResidualStream, row_index: Optional[torch.Tensor] = None,
               buffer: str = "normed", out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
         """Fold what waits on the stream into the residual and return the normed rows.

@@ -1,0 +1,90 @@
+"""Layers that run from the recorded calls of a layer like them: the same bits and the same number of launches as layers
+that run one by one, in prompts, mixed steps and both engines, and not for layers that differ."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def build(dtype, layers=6, window=None, seed=0):
+    from socrates_b200 import Engine
+    from socrates_b200.config import config_from_dict
+    from socrates_b200.engine.model import Model
+    config = config_from_dict({
+        "architectures": ["Qwen3ForCausalLM"], "vocab_size": 300, "hidden_size": 256, "intermediate_size": 384,
+        "num_hidden_layers": layers, "num_attention_heads": 4, "num_key_value_heads": 2, "head_dim": 64,
+        "rms_norm_eps": 1e-6, "rope_theta": 1e4, "tie_word_embeddings": False, "max_position_embeddings": 4096,
+        "sliding_window": window, "use_sliding_window": window is not None, "max_window_layers": 3})
+    model = Model(config.plan())
+    g = torch.Generator().manual_seed(seed)
+    tensors = {}
+    for name, spec in model.parameters().items():
+        t = torch.randn(spec.shape, generator=g)
+        tensors[name] = (1 + 0.1 * t if len(spec.shape) == 1 else (0.05 * t).to(dtype)).to(DEV)
+    model.bind(tensors, dtype)
+    return Engine((config, model), device="cuda:0", dtype=dtype, block_size=16, max_batch=4, max_len=2048, token_budget=600,
+                  num_blocks=400)
+
+
+def steps(engine):
+    """Logits of a prompt, of its second portion beside two new prompts, and of a step that mixes both kinds."""
+    from socrates_b200.engine.runner import StepEntry
+    g = torch.Generator().manual_seed(5)
+    ids = lambda n: torch.randint(0, 300, (n,), generator=g).tolist()
+    cache, out, at = engine.cache, [], {}
+    for row in range(4):
+        cache.assign(row)
+    for portions in ([(0, 70)], [(0, 200), (1, 9), (2, 130)], [(0, 1), (1, 1), (3, 300), (2, 1)], [(0, 5), (1, 2)]):
+        entries = []
+        for row, n in portions:
+            start = at.get(row, 0)
+            assert cache.reserve(row, start + n)
+            entries.append(StepEntry(row, ids(n), start, [n - 1]))
+        out.append(engine.runner.step(entries).logits.clone())
+        for row, n in portions:
+            at[row] = at.get(row, 0) + n
+            cache.commit(row, at[row])
+    return out, engine.runner.kernel_launches
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("window", [None, 40])
+def test_recorded_layers_give_the_same_bits(dtype, window, monkeypatch):
+    from socrates_b200.engine.model import Model
+    from socrates_b200.kernels.layer_calls import Recording
+    runs = []
+    run = Recording.run
+    monkeypatch.setattr(Recording, "run", lambda self, a: (runs.append(1), run(self, a))[1])
+    got, launches = steps(build(dtype, window=window))
+    assert len(runs) >= 4                               # every step had layers that ran from another's calls
+    monkeypatch.setattr(Model, "_like_another", lambda *a: False)
+    want, plain = steps(build(dtype, window=window))
+    assert launches == plain
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
+def test_a_layer_with_a_tensor_of_another_type_runs_by_itself(monkeypatch):
+    """One float32 matrix in a bfloat16 engine goes through another kernel."""
+    from socrates_b200.engine.model import Model
+    from socrates_b200.parts.linear import Linear
+
+    def odd():
+        engine = build(torch.bfloat16)
+        layer = engine.model.layers[3]
+        layer.mixer.o = Linear(layer.mixer.o.weight.float())
+        return engine
+    got, launches = steps(odd())
+    monkeypatch.setattr(Model, "_like_another", lambda *a: False)
+    want, plain = steps(odd())
+    assert launches == plain and all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+def test_words_per_entry_point():
+    from socrates_b200.kernels.layer_calls import ENTRIES
+    from socrates_b200.kernels.library import _SIGNATURES, library
+    for name, number in ENTRIES.items():
+        assert library().sb_run_calls_arity(number) == len(_SIGNATURES[name]), name
+    assert library().sb_run_calls_arity(len(ENTRIES)) == -1
