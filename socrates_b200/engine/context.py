@@ -183,14 +183,23 @@ class StepContext:
         As many parts as there are places (two blocks an SM up to 128 rows, one beyond), at least four K blocks each; it
         takes three parts to beat the other kernels.  Measured (us, before / so): 187 rows: 2,560 x 4,096 16.8 / 11.4,
         2,560 x 9,728 26.1 / 16.7, 6,144 x 2,560 16.8 / 13.3, 5,120 x 25,600 70.8 / 59.5, 4,096 x 12,288 30.5 / 28.7; 72
-        rows: 13.0 / 8.1, 21.7 / 12.9, 12.1 / 9.7, 56.0 / 54.4, 27.0 / 24.1.  256 columns are a heavier tile: there only
-        where nine tenths of the SMs get a block (2,560 x 9,728 26.5 / 19.3, but 4,096 x 12,288 31.8 / 33.8)."""
+        rows: 13.0 / 8.1, 21.7 / 12.9, 12.1 / 9.7, 56.0 / 54.4, 27.0 / 22.6.  256 columns are a heavier tile: there only
+        where nine tenths of the SMs get a block (2,560 x 9,728 26.5 / 19.3, but 4,096 x 12,288 31.8 / 33.8).
+        A short product that narrows follows attention, whose blocks hold a third of the SMs: with one block an SM its
+        blocks should all find room beside them, so that their first weights are there when attention ends (4,096 x 4,096
+        in 128 blocks ended 27 us after it in the 8B step, the kernel before in 13), and there must be four parts of it."""
         if not 64 < M <= 256 or not self.uses_tensor_cores(x_dtype, w):
             return 0
         N, K = w.shape
         tiles = -(-N // 128)
         parts = min((2 if M <= 128 else 1) * self.num_sms // tiles, -(-K // 64) // 4, 14)
-        if parts < 3 or (M > 192 and 10 * tiles * parts < 9 * self.num_sms):
+        if M > 192 and 10 * tiles * parts < 9 * self.num_sms:
+            return 0
+        if M > 128 and N <= K < 8192:
+            parts = min(parts, 7 * self.num_sms // 10 // tiles)
+            if parts < 4:
+                return 0
+        if parts < 3:
             return 0
         return ops.gemm_tcgen05_splits(K, parts)
 
