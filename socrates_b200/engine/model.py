@@ -58,6 +58,10 @@ class Model:
             if what not in kinds:
                 kinds.append(what)
             self._kind_of_layer.append(kinds.index(what))
+        # layers of the same kind that run after each order entry: a recording pays from the second on (the last layer's
+        # products are followed by another matrix)
+        self._alike_after = [sum(self._kind_of_layer[later.layer] == self._kind_of_layer[e.layer]
+                                 for later in plan.order[i + 1:]) for i, e in enumerate(plan.order)]
         self.final_norm = build_part("norm", plan.final_norm, plan.final_norm.name)
         self.head = build_part("head", plan.head, plan.head.name)
         self.dtype: Optional[torch.dtype] = None
@@ -128,6 +132,8 @@ class Model:
                 or not waits.plain or stream.add_rows is not None or stream.add_vec is not None
                 or stream.streams is not None):
             return False
+        if not recordings and self._alike_after[i] < 2:
+            return False
         tensors = layer.replay_tensors()
         own = {t.data_ptr() for t in tensors}
         after = []                                      # which product follows each: one of the layer's own, or another's
@@ -145,7 +151,7 @@ class Model:
             known[0].run(addresses)
             stream.pending = known[1]
             return True
-        if known is not None:
+        if known is not None or self._alike_after[i] < 2:
             return False
         recording = Recording(addresses)
         with recording:
