@@ -21,8 +21,8 @@ namespace {
 //   EPI = 1: the weight rows interleave gate and up (row 2f = gate_f, row 2f+1 = up_f);
 //            C[m, f] = up * silu(gate), C has N/2 columns (SiLU*mul fused into the product).
 //
-// ISSUERS = 2 (tile widths below 256, where one thread's rate of about one product every 80 ns,
-// not the tensor core, sets the pace): a seventh warp issues too.  Each of the two threads issues
+// ISSUERS = 2 (tile widths below 256, where one warp's waits, products and commits per K block, not the
+// tensor core, set the pace): a seventh warp issues too.  Each of the two warps issues
 // half of every K block's products into an accumulator of its own (columns BN.. beside the
 // first), and the epilogue adds the two.  Where four such accumulators do not fit into the 512
 // columns, a tile's main loop waits for the epilogue of the tile before it.

@@ -55,8 +55,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
 // A warp that issues tensor-core products walks its loop as a WHOLE and lets one elected lane execute the products and
 // commits.  tcgen05.mma takes its descriptors from uniform registers: inside a branch that only one lane takes, nothing is
 // known to be uniform and every operand of every product is moved there first, which made one product about 80 ns (150
-// clocks) whatever its size.  Walked whole, the products of a 2,048-row step: 62 -> 53 us (2,560 x 4,096 in equal shares), 158 -> 152
-// (19,456 x 2,560), and prompt attention of 2,048 tokens 100 -> 81 us.  The lane that elect.sync picks for a full mask is always the same, as commits need it to be.
+// clocks) whatever its size.  Walked whole, the products of a 2,048-row step: 62 -> 53 us (2,560 x 4,096 in equal
+// shares), 158 -> 152 (19,456 x 2,560), and prompt attention of 2,048 tokens 100 -> 81 us.  The lane that elect.sync picks
+// for a full mask is always the same, as commits need it to be.
 __device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); }
 __device__ __forceinline__ bool elect_one() {
     uint32_t one;
