@@ -45,7 +45,8 @@ template <int MT> constexpr int few_smem() { return GROUPS * RING * few_stage_fl
 
 template <int MT>
 __global__ void __launch_bounds__(NTHR)
-gemm_f32_few_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W, int M, int N, int K) {
+gemm_f32_few_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W, int M, int N, int K,
+                    int w_older) {
     sb::pdl_launch_dependents();
     extern __shared__ __align__(16) float smem[];
     constexpr int STAGE = few_stage_floats<MT>();
@@ -75,11 +76,15 @@ gemm_f32_few_kernel(float* __restrict__ C, const float* __restrict__ A, const fl
             copy16(smem_addr(st + m * PIECE + 4 * p), ok ? A + (size_t)m * K + k0 + 4 * p : A, ok ? 16 : 0);
         }
     };
-    // weights are older than the kernel before this one; activations are not
+    // A, and W too unless the caller says that it is older, may come from the kernel before this one
+    auto first_w = [&] {
 #pragma unroll
-    for (int i = 0; i < RING - 1; ++i)
-        if (begin + i < end) load_w(begin + i);
+        for (int i = 0; i < RING - 1; ++i)
+            if (begin + i < end) load_w(begin + i);
+    };
+    if (w_older) first_w();
     sb::pdl_wait();
+    if (!w_older) first_w();
 #pragma unroll
     for (int i = 0; i < RING - 1; ++i) {
         if (begin + i < end) load_a(begin + i);
@@ -147,7 +152,7 @@ __device__ __forceinline__ unsigned long long twice(float x) {
 template <bool CLUSTER>
 __global__ void __launch_bounds__(NTHR, 2)
 gemm_f32_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W, int M, int N, int K,
-                     int row_tiles) {
+                     int row_tiles, int w_older) {
     sb::pdl_launch_dependents();
     extern __shared__ __align__(16) float smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -185,8 +190,9 @@ gemm_f32_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const f
             ra[4 + p] = ok ? *reinterpret_cast<const float4*>(a1 + k0 + 4 * p) : zero;
         }
     };
-    if (begin < end) fetch_w(begin);    // weights are older than the kernel before this one
+    if (w_older && begin < end) fetch_w(begin);             // W as in the kernel above
     sb::pdl_wait();
+    if (!w_older && begin < end) fetch_w(begin);
     if (begin < end) fetch_a(begin);
     const int tx = lane & 7, ty = lane >> 3;                // columns 4 tx + 32 h + j, rows 4 ty + 16 i + e
     unsigned long long acc[8][8];                           // [pairs of rows: 2 i + e / 2][columns: 4 h + j]
@@ -285,7 +291,8 @@ gemm_f32_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const f
     }
 }
 
-template <int MT> int launch_few(float* C, const float* A, const float* W, int M, int N, int K, cudaStream_t stream) {
+template <int MT>
+int launch_few(float* C, const float* A, const float* W, int M, int N, int K, int w_older, cudaStream_t stream) {
     static sb::OncePerDevice once_per_device;
     bool& configured = once_per_device.flag();
     if (!configured) {
@@ -293,7 +300,8 @@ template <int MT> int launch_few(float* C, const float* A, const float* W, int M
         if (e != cudaSuccess) { sb_set_error("gemm_f32: %s", cudaGetErrorString(e)); return (int)e; }
         configured = true;
     }
-    sb::launch(gemm_f32_few_kernel<MT>, dim3((N + COLS - 1) / COLS), dim3(NTHR), few_smem<MT>(), stream, C, A, W, M, N, K);
+    sb::launch(gemm_f32_few_kernel<MT>, dim3((N + COLS - 1) / COLS), dim3(NTHR), few_smem<MT>(), stream, C, A, W, M, N, K,
+               w_older);
     return 0;
 }
 
@@ -309,11 +317,12 @@ bool gemm_f32_takes(const void* C, const void* A, const void* W, int M, int N, i
     return K % 4 == 0 && (bits & 15) == 0 && blocks <= 0x7fffffffLL;
 }
 
-int gemm_f32(float* C, const float* A, const float* W, int M, int N, int K, cudaStream_t stream) {
-    if (M <= 1) return launch_few<1>(C, A, W, M, N, K, stream);
-    if (M <= 2) return launch_few<2>(C, A, W, M, N, K, stream);
-    if (M <= 4) return launch_few<4>(C, A, W, M, N, K, stream);
-    if (M <= 8) return launch_few<8>(C, A, W, M, N, K, stream);
+// `w_older`: nothing that the kernel before this one on the stream writes is in W (see sb_gemm_simt).
+int gemm_f32(float* C, const float* A, const float* W, int M, int N, int K, int w_older, cudaStream_t stream) {
+    if (M <= 1) return launch_few<1>(C, A, W, M, N, K, w_older, stream);
+    if (M <= 2) return launch_few<2>(C, A, W, M, N, K, w_older, stream);
+    if (M <= 4) return launch_few<4>(C, A, W, M, N, K, w_older, stream);
+    if (M <= 8) return launch_few<8>(C, A, W, M, N, K, w_older, stream);
     static sb::OncePerDevice once_per_device;
     bool& configured = once_per_device.flag();
     if (!configured) {
@@ -328,9 +337,10 @@ int gemm_f32(float* C, const float* A, const float* W, int M, int N, int K, cuda
     // blocks then.
     if (tiles < 888)
         sb::launch_cluster(gemm_f32_tile_kernel<true>, dim3(tiles * GROUPS), dim3(NTHR), TILE_SMEM, stream, dim3(GROUPS), C, A, W,
-                           M, N, K, row_tiles);
+                           M, N, K, row_tiles, w_older);
     else
-        sb::launch(gemm_f32_tile_kernel<false>, dim3(tiles), dim3(NTHR), TILE_SMEM, stream, C, A, W, M, N, K, row_tiles);
+        sb::launch(gemm_f32_tile_kernel<false>, dim3(tiles), dim3(NTHR), TILE_SMEM, stream, C, A, W, M, N, K, row_tiles,
+                   w_older);
     return 0;
 }
 

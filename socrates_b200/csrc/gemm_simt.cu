@@ -10,7 +10,7 @@ using namespace sb;
 
 namespace sb {                          // gemm_f32.cu
 bool gemm_f32_takes(const void* C, const void* A, const void* W, int M, int N, int K);
-int gemm_f32(float* C, const float* A, const float* W, int M, int N, int K, cudaStream_t stream);
+int gemm_f32(float* C, const float* A, const float* W, int M, int N, int K, int w_older, cudaStream_t stream);
 }
 
 namespace {
@@ -84,15 +84,17 @@ void launch(void* C, const void* A, const void* W, int M, int N, int K, int spli
 
 }  // namespace
 
+// `w_older`: W is complete before the kernel that precedes this one on the stream starts (a bound weight within a step), so it
+// may be read before that kernel has ended.
 extern "C" int sb_gemm_simt(void* C, const void* A, const void* W, int M, int N, int K, int a_dtype,
-                            int w_dtype, int c_dtype, int splits, cudaStream_t stream) {
+                            int w_dtype, int c_dtype, int splits, int w_older, cudaStream_t stream) {
     SB_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm_simt: bad sizes M=%d N=%d K=%d", M, N, K);
     SB_REQUIRE(splits >= 1 && splits <= 64, "gemm_simt: splits=%d is outside 1..64", splits);
     SB_REQUIRE(splits == 1 || c_dtype == SB_F32, "gemm_simt: partial sums of a split product are float32");
     SB_REQUIRE((M + BM - 1) / BM <= 65535, "gemm_simt: M=%d is too large", M);
     if (M == 0) return 0;
     if (a_dtype == SB_F32 && w_dtype == SB_F32 && c_dtype == SB_F32 && splits == 1 && sb::gemm_f32_takes(C, A, W, M, N, K)) {
-        const int rc = sb::gemm_f32((float*)C, (const float*)A, (const float*)W, M, N, K, stream);
+        const int rc = sb::gemm_f32((float*)C, (const float*)A, (const float*)W, M, N, K, w_older, stream);
         if (rc != 0) return rc;
         SB_LAUNCH_CHECK();
     }

@@ -16,7 +16,7 @@
 extern "C" {
 int sb_add_rmsnorm(float*, const float*, int, long long, const float*, void*, const int*, int, int, float, int, cudaStream_t);
 int sb_gemm_tcgen05(void*, const void*, const void*, int, int, int, int, int*, int*, int, int, const void*, long long, cudaStream_t);
-int sb_gemm_simt(void*, const void*, const void*, int, int, int, int, int, int, int, cudaStream_t);
+int sb_gemm_simt(void*, const void*, const void*, int, int, int, int, int, int, int, int, cudaStream_t);
 int sb_qk_norm_rope_kvwrite(const void*, const float*, int, long long, void*, void*, void*, const float*, const float*,
                             const float*, int, const int*, const int*, const int*, int, int, float, int, int, int, int, int, int,
                             int, int, int, const float*, int, float, int, int, int, float, float*, cudaStream_t);

@@ -127,7 +127,8 @@ class StepContext:
         self.num_sms = num_sms
         self.status = status                # int32 device word the tensor-core kernels report to
         self.token_feedback = token_feedback   # int32 device tokens that ids -1 - j stand for (see ops.embed)
-        self.weight_successor: Dict[int, torch.Tensor] = {}   # set by the model: address -> next weights
+        # set by the model: address of each of its streamed weights -> the next one's tensor (None after the last)
+        self.weight_successor: Dict[int, Optional[torch.Tensor]] = {}
         self.l2_prefetch_bytes = _l2_prefetch_budget()
         self.dependent_launch = True        # set by the model: whether the step's kernels are launched dependently
         self.after_run = None               # callable(order index, stream) after every layer run (for inspection)
@@ -254,7 +255,8 @@ class StepContext:
         else:
             if epilogue:
                 raise ValueError("the fused epilogue exists only in the tensor-core kernel")
-            ops.gemm_simt(out, x, w, splits=S)
+            # a matrix of the model's own was bound before the step; any other may come from the kernel before this one
+            ops.gemm_simt(out, x, w, splits=S, w_older=w.data_ptr() in self.weight_successor)
 
     def _next_weights(self, w: torch.Tensor, splits: int):
         nxt = self.weight_successor.get(w.data_ptr())

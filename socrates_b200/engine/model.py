@@ -95,8 +95,10 @@ class Model:
         for e in self.plan.order:
             order.extend(getattr(self.layers[e.layer], "streamed_weights", list)())
         order.extend(getattr(self.head, "streamed_weights", list)())
-        self.weight_successor: Dict[int, torch.Tensor] = {}
-        for w, nxt in zip(order, order[1:]):
+        # (The list keeps them: an address in the map is never another tensor's.)
+        self._streamed = order
+        self.weight_successor: Dict[int, Optional[torch.Tensor]] = {}
+        for w, nxt in zip(order, [*order[1:], None]):
             self.weight_successor.setdefault(w.data_ptr(), nxt)
 
     # ------------------------------------------------------------------ cache

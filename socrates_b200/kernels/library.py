@@ -37,7 +37,7 @@ _SIGNATURES = {
     "sb_silu_mul": [P, P, I, I, I, I, I, P],
     "sb_sample": [P, P, P, P, P, I, I, P, P],
     "sb_sample_slices": [I],
-    "sb_gemm_simt": [P, P, P, I, I, I, I, I, I, I, P],
+    "sb_gemm_simt": [P, P, P, I, I, I, I, I, I, I, I, P],
     "sb_attention_simt": [P, P, P, P, P, P, P, I, P, P, I, I, I, I, I, I, F, I, I, P],
     "sb_gemm_tcgen05": [P, P, P, I, I, I, I, P, P, I, I, P, LL, P],
     "sb_gemm_tcgen05_splits": [I, I],

@@ -236,10 +236,12 @@ def sample(out: torch.Tensor, logits: torch.Tensor, temperature: Optional[torch.
                              M, V, _ptr(scratch), _stream()), "sample")
 
 
-def gemm_simt(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, splits: int = 1) -> None:
+def gemm_simt(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, splits: int = 1, w_older: bool = False) -> None:
     """out = a @ w.T on the CUDA cores with float32 accumulation.
 
-    a [M, K], w [N, K]; out [M, N], or float32 [splits, M, N] partial sums.
+    a [M, K], w [N, K]; out [M, N], or float32 [splits, M, N] partial sums.  `w_older`: `w` was complete before the
+    kernel that precedes this one on the stream started (a bound weight within a step); the kernel may then fetch
+    it while that one still runs.
     """
     M, K = a.shape
     N = w.shape[0]
@@ -251,7 +253,7 @@ def gemm_simt(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, splits: int =
         _want(out, "out", torch.float32, (splits, M, N))
     lib = library()
     check(lib, lib.sb_gemm_simt(_ptr(out), _ptr(a), _ptr(w), M, N, K, _code(a.dtype), _code(w.dtype),
-                                _code(out.dtype), splits, _stream()), "gemm_simt")
+                                _code(out.dtype), splits, int(w_older), _stream()), "gemm_simt")
 
 
 def attention_simt(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,

@@ -30,3 +30,19 @@ def test_gemm_f32(ops, N, K):
         assert bool(((out.double() - exact[:M]).abs() <= bound[:M]).all()), M
         whole = out if whole is None else whole
         assert torch.equal(out, whole[:M]), M
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 2560, 1024), (8, 2560, 1024), (70, 2560, 1024), (64, 57600, 64)])
+def test_a_matrix_that_the_kernel_before_writes(ops, M, N, K):
+    """w is the result of the kernel right before this one on the stream, which lets its successor start early: nothing of
+    w may be read before that kernel has ended (1 and 8 rows, tiles in clusters, whole tiles)."""
+    a, x, y = (rand(n, k, dtype=torch.float32, seed=s) for n, k, s in ((M, K, 1), (N, 256, 2), (K, 256, 3)))
+    w, out, want = torch.empty(N, K, device=DEV), torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    ops.gemm_simt(w, x, y)
+    torch.cuda.synchronize()
+    ops.gemm_simt(want, a, w.clone(), w_older=True)
+    for _ in range(8):
+        w.fill_(float("nan"))
+        ops.gemm_simt(w, x, y)
+        ops.gemm_simt(out, a, w)
+        assert torch.equal(out, want)
