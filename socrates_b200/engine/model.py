@@ -15,7 +15,7 @@ import torch
 from ..cache.manager import CacheNeeds
 from ..config.plan import ModelPlan
 from ..kernels import ops
-from ..kernels.layer_calls import Recording
+from ..kernels.layer_calls import Recording, layer_facts
 from ..parts import ParamSpec, ResidualStream, build_part
 from ..parts.base import _REGISTRIES
 from .context import CacheView, StepContext
@@ -47,21 +47,16 @@ class Model:
                 if hasattr(p, "prefers_shares"):
                     dealers.setdefault((p.Hq, p.Hkv, p.D, p.window), p)
         self._key_dealers = list(dealers.values())
-        # layers of equal specs, by number (see _like_another); -1: a layer that does not say what its kernels are given
+        # layers of equal specs that run after each order entry: a recording pays from the second on (the last layer's
+        # products are followed by another matrix).  Whether layers are alike is for _like_another to see.
         kinds: List = []
-        self._kind_of_layer: List[int] = []
-        for spec, layer in zip(plan.layers, self.layers):
+        for spec in plan.layers:
             what = (spec.arrangement, spec.norms, spec.mixer, spec.feed_forward, spec.params)
-            if "replay_tensors" not in type(layer).__dict__ or layer.replay_parts() is None:
-                self._kind_of_layer.append(-1)
-                continue
-            if what not in kinds:
-                kinds.append(what)
-            self._kind_of_layer.append(kinds.index(what))
-        # layers of the same kind that run after each order entry: a recording pays from the second on (the last layer's
-        # products are followed by another matrix)
-        self._alike_after = [sum(self._kind_of_layer[later.layer] == self._kind_of_layer[e.layer]
-                                 for later in plan.order[i + 1:]) for i, e in enumerate(plan.order)]
+            kinds.append(next((k for k, other in enumerate(plan.layers[:len(kinds)])
+                               if what == (other.arrangement, other.norms, other.mixer, other.feed_forward, other.params)),
+                              len(kinds)))
+        self._alike_after = [sum(kinds[later.layer] == kinds[e.layer] for later in plan.order[i + 1:])
+                             for i, e in enumerate(plan.order)]
         self.final_norm = build_part("norm", plan.final_norm, plan.final_norm.name)
         self.head = build_part("head", plan.head, plan.head.name)
         self.dtype: Optional[torch.dtype] = None
@@ -125,18 +120,19 @@ class Model:
         """Run order entry i from the calls of an earlier layer of this step that it is like, or record its own; False: it
         is to run as any layer.  For steps that launch their kernels from here (a recorded graph needs none of this): a
         prompt portion of 187 tokens through 18 layers of the 4B shape took the host 2.9 ms in single launches, longer
-        than the GPU.  What makes layers alike is looked at in every step: their specs, the shape, type and alignment of
-        every tensor, what the product after each is, the pages' table and what waits on the stream."""
-        layer_index = self.plan.order[i].layer
-        layer = self.layers[layer_index]
+        than the GPU.  What makes layers alike is looked at in every step: every class, function and constant in them, the
+        shape, type and alignment of every tensor, what the product after each is, the pages' table and what waits
+        on the stream."""
+        layer = self.layers[self.plan.order[i].layer]
         waits = stream.pending
-        if (ctx.host_batch is None or ctx.after_run is not None or self._kind_of_layer[layer_index] < 0 or waits is None
-                or not waits.plain or stream.add_rows is not None or stream.add_vec is not None
-                or stream.streams is not None):
+        if (ctx.host_batch is None or ctx.after_run is not None or waits is None or not waits.plain
+                or stream.add_rows is not None or stream.add_vec is not None or stream.streams is not None):
             return False
         if not recordings and self._alike_after[i] < 2:
             return False
-        tensors = layer.replay_tensors()
+        facts, tensors = [], []
+        if not layer_facts(layer, facts, tensors):
+            return False
         own = {t.data_ptr() for t in tensors}
         after = []                                      # which product follows each: one of the layer's own, or another's
         for w in layer.streamed_weights():
@@ -145,8 +141,9 @@ class Model:
             if nxt is not None and not after[-1]:
                 tensors.append(nxt)
         tensors.extend(view.pools())
-        key = (self._kind_of_layer[layer_index], tuple(after), view.block_table().data_ptr(), waits.partial.data_ptr(),
-               waits.partial.shape, tuple([(t.shape, t.dtype, t.is_contiguous(), t.data_ptr() & 127) for t in tensors]))
+        table = view.block_table()
+        key = (tuple(facts), tuple(after), table.data_ptr(), table.shape, waits.partial.data_ptr(), waits.partial.shape,
+               tuple([(t.shape, t.dtype, t.is_contiguous(), t.data_ptr() & 127) for t in tensors]))
         addresses = [t.data_ptr() for t in tensors]
         known = recordings.get(key)
         if known is not None and known[0].usable:

@@ -5,13 +5,17 @@ pages.  `Recording` collects a layer's calls as the words that `sb_run_calls` ta
 the places that hold the layer's own addresses; `run` fills in another layer's and launches all of it in one call.  A
 recording lives for one step: nothing is kept from one step to the next, and buffers, scratch, sizes and the stream are the
 step's.
+
+Which layers are alike is read off the layers themselves in every step (`layer_facts`): a class says with `@replayable`
+what its calls depend on.
 """
 
 from __future__ import annotations
 
 import ctypes
 import struct
-from typing import Dict, List, Optional, Sequence, Tuple
+from operator import attrgetter
+from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
 import torch
@@ -25,6 +29,52 @@ ENTRIES = {"sb_add_rmsnorm": 0, "sb_gemm_tcgen05": 1, "sb_gemm_simt": 2, "sb_qk_
 # host-only questions that a layer may ask while it is recorded
 _QUESTIONS = ("_supports", "_splits", "_parts", "_shares", "_kernels", "_blocks_per_sm", "sb_last_error",
               "sb_set_dependent_launch")
+
+
+# class -> (method, its function, an instance's constants, its tensors, those it may lack, the parts inside it)
+_REPLAYABLE: Dict[type, Tuple[str, Callable, Callable, Callable, Callable, Callable]] = {}
+
+
+def replayable(method: str, constants: Sequence[str] = (), tensors: Sequence[str] = (), optional: Sequence[str] = (),
+               parts: Callable = lambda self: ()):
+    """Class decorator: what `method` launches depends on the instance through the attributes named here (`tensors`, and
+    `optional` ones that may be None) and the `parts` inside it alone.  It holds for the very class (a subclass may launch
+    other things) and for the very function."""
+    def getter(names):
+        get = attrgetter(*names) if names else None
+        return (lambda self: ()) if get is None else get if len(names) > 1 else (lambda self: (get(self),))
+
+    def mark(cls):
+        _REPLAYABLE[cls] = (method, cls.__dict__[method], getter(constants), getter(tensors), getter(optional), parts)
+        return cls
+    return mark
+
+
+def layer_facts(part, facts: list, tensors: list) -> bool:
+    """Append what the calls of `part` depend on: `tensors` whose addresses stand in them, and everything else to `facts`
+    (two layers with equal facts make the same calls but for these addresses).  False: that is not known, because
+    something in the layer is no replayable class or lacks a tensor, or a method was replaced or wrapped, on the class or on
+    the instance."""
+    known = _REPLAYABLE.get(type(part))
+    if known is None:
+        return False
+    method, function, constants, own, optional, parts = known
+    if type(part).__dict__.get(method) is not function or method in part.__dict__:
+        return False
+    facts.append(type(part))
+    facts.append(constants(part))
+    for t in own(part):
+        if t is None:
+            return False
+        tensors.append(t)
+    for t in optional(part):
+        facts.append(t is None)
+        if t is not None:
+            tensors.append(t)
+    for inner in parts(part):
+        if not layer_facts(inner, facts, tensors):
+            return False
+    return True
 
 
 class _Recorder:

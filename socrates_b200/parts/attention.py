@@ -22,6 +22,7 @@ import torch
 
 from ..cache.manager import CacheNeeds, PagedKVSpec
 from ..kernels import ops
+from ..kernels.layer_calls import replayable
 from .base import Branch, ParamSpec, Part, build_part, register_part
 from .linear import Linear
 
@@ -145,6 +146,8 @@ def paged_attention(ctx, out, q, k_pool, v_pool, table, num_heads: int, scale: f
                            window, NP, part_o, part_ml)
 
 
+@replayable("forward", constants=("Hq", "Hkv", "D", "scale", "qk_norm_eps", "window"), optional=("q_gain", "k_gain"),
+            parts=lambda self: (self.position, self.qkv, self.o))
 class GQAAttention(Part):
     def __init__(self, spec, name):
         super().__init__(spec, name)
@@ -194,10 +197,6 @@ class GQAAttention(Part):
     def streamed_weights(self):
         """The weight matrices in the order in which forward() reads them."""
         return [self.qkv.weight, self.o.weight]
-
-    def replay_tensors(self):
-        inv_freq, _ = self.position.tables(self.o.weight.device)
-        return [t for t in (self.qkv.weight, self.o.weight, self.q_gain, self.k_gain, inv_freq) if t is not None]
 
     def prefers_shares(self, lengths: Sequence[int], num_sms: int) -> bool:
         """Whether a decode step over rows of so many keys should deal them in equal shares (attention_balanced.cu)

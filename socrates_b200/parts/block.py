@@ -12,10 +12,12 @@ from typing import Dict, Mapping
 
 import torch
 
+from ..kernels.layer_calls import replayable
 from .base import ParamSpec, ResidualStream, build_part, register_part
 from .norm import fold_and_norm
 
 
+@replayable("forward", parts=lambda self: (*self.norms, self.mixer, self.feed_forward))
 class PreNormBlock:
     def __init__(self, layer_spec):
         if len(layer_spec.norms) != 2:
@@ -51,16 +53,6 @@ class PreNormBlock:
         """Weight matrices in the order in which forward() streams them (optional for a part)."""
         return [*getattr(self.mixer, "streamed_weights", list)(),
                 *getattr(self.feed_forward, "streamed_weights", list)()]
-
-    def replay_parts(self):
-        """The layer's parts if its kernels are given nothing of the layer's own but `replay_tensors()` (and its pages), or
-        None: another layer of the same specs then makes the same calls with its own tensors in these places
-        (kernels/layer_calls.py).  The very class of a part must say so: a subclass may launch other things."""
-        parts = self.parts()
-        return parts if all("replay_tensors" in type(p).__dict__ for p in parts) else None
-
-    def replay_tensors(self):
-        return [t for p in self.parts() for t in p.replay_tensors()]
 
     def forward(self, ctx, stream: ResidualStream, cache) -> None:
         h = self.norms[0].apply(ctx, stream)

@@ -14,10 +14,12 @@ from typing import Dict, Mapping, Optional
 import torch
 
 from ..kernels import ops
+from ..kernels.layer_calls import replayable
 from .base import Branch, ParamSpec, Part, register_part
 from .linear import Linear
 
 
+@replayable("forward", constants=("inter", "act"), parts=lambda self: (self.gate_up, self.down))
 class SwiGLU(Part):
     def __init__(self, spec, name):
         super().__init__(spec, name)
@@ -47,9 +49,6 @@ class SwiGLU(Part):
 
     def streamed_weights(self):
         """The weight matrices in the order in which forward() reads them."""
-        return [self.gate_up.weight, self.down.weight]
-
-    def replay_tensors(self):
         return [self.gate_up.weight, self.down.weight]
 
     def forward(self, ctx, x: torch.Tensor) -> Branch:

@@ -10,9 +10,10 @@ from __future__ import annotations
 
 import torch
 
-from ..kernels import ops
+from ..kernels.layer_calls import replayable
 
 
+@replayable("__call__", constants=("out_features", "in_features"), tensors=("weight",))
 class Linear:
     def __init__(self, weight: torch.Tensor):
         if weight.dim() != 2:

@@ -24,6 +24,7 @@ from typing import Dict, Mapping, Optional
 import torch
 
 from ..kernels import ops
+from ..kernels.layer_calls import replayable
 from .base import ParamSpec, Part, ResidualStream, register_part
 
 
@@ -53,6 +54,7 @@ def fold_and_norm(stream: ResidualStream, gain: Optional[torch.Tensor], out: Opt
         stream.rows = None
 
 
+@replayable("apply", constants=("dim", "eps"), tensors=("gain",))
 class RMSNorm(Part):
     def __init__(self, spec, name):
         super().__init__(spec, name)
@@ -68,9 +70,6 @@ class RMSNorm(Part):
     def bind(self, tensors: Mapping[str, torch.Tensor], dtype) -> None:
         g = tensors[self.tensor]
         self.gain = (g + self.offset).contiguous() if self.offset else g
-
-    def replay_tensors(self):
-        return [self.gain]
 
     def apply(self, ctx, stream: ResidualStream, row_index: Optional[torch.Tensor] = None,
               buffer: str = "normed", out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:

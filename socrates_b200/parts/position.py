@@ -32,9 +32,11 @@ from typing import Optional, Tuple
 
 import torch
 
+from ..kernels.layer_calls import replayable
 from .base import Part, register_part
 
 
+@replayable("tables", constants=("rotary_dim", "magnitude"), tensors=("_table",))
 class Rotary(Part):
     """inv_freq_j = theta^(-2j/D), j < D/2, in float32 exactly as the reference builds
     it (model/qwen/qwen_kv_cont.py:56-64)."""
@@ -112,6 +114,7 @@ class Rotary(Part):
         return self._table, self.rotary_dim
 
 
+@replayable("tables", constants=("magnitude",), tensors=("_table",))
 class NoPosition(Part):
     """No rotation: the mixer's kernel passes every dim through."""
 

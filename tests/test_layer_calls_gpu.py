@@ -82,6 +82,34 @@ def test_a_layer_with_a_tensor_of_another_type_runs_by_itself(monkeypatch):
     assert launches == plain and all(torch.equal(a, b) for a, b in zip(got, want))
 
 
+@pytest.mark.parametrize("change", [
+    lambda layer: setattr(layer.mixer, "window", 24), lambda layer: setattr(layer.mixer, "scale", 0.3),
+    lambda layer: setattr(layer.norms[1], "eps", 0.5), lambda layer: setattr(layer.mixer.position, "magnitude", 1.5)])
+def test_a_layer_that_was_changed_after_it_was_built(change, monkeypatch):
+    from socrates_b200.engine.model import Model
+
+    def odd():
+        engine = build(torch.bfloat16)
+        change(engine.model.layers[3])
+        return engine
+    got, launches = steps(odd())
+    monkeypatch.setattr(Model, "_like_another", lambda *a: False)
+    want, plain = steps(odd())
+    assert launches == plain and all(torch.equal(a, b) for a, b in zip(got, want))
+    same, _ = steps(build(torch.bfloat16))
+    assert not torch.equal(got[0], same[0])             # the change shows at all
+
+
+def test_a_wrapped_layer_is_called_in_every_step():
+    engine, calls = build(torch.bfloat16), []
+    layer = engine.model.layers[3]
+    forward = layer.mixer.forward
+    layer.mixer.forward = lambda *a: (calls.append(1), forward(*a))[1]
+    got, _ = steps(engine)
+    same, _ = steps(build(torch.bfloat16))
+    assert len(calls) == 4 and all(torch.equal(a, b) for a, b in zip(got, same))
+
+
 def test_words_per_entry_point():
     from socrates_b200.kernels.layer_calls import ENTRIES
     from socrates_b200.kernels.library import _SIGNATURES, library

@@ -37,3 +37,72 @@ def test_every_streamed_weight_is_known():
     weights = [w for layer in model.layers for w in layer.streamed_weights()] + model.head.streamed_weights()
     assert len(weights) == 9 and [w.data_ptr() for w in weights] == list(model.weight_successor)
     assert model.weight_successor[weights[-1].data_ptr()] is None
+
+
+# ---------------------------------------------------------------------- layers that run from another's recorded calls
+def qwen3(layers=3):
+    from socrates_b200.config import config_from_dict
+    from socrates_b200.engine.model import Model
+    model = Model(config_from_dict({
+        "architectures": ["Qwen3ForCausalLM"], "vocab_size": 32, "hidden_size": 32, "intermediate_size": 48,
+        "num_hidden_layers": layers, "num_attention_heads": 2, "num_key_value_heads": 1, "head_dim": 16, "rms_norm_eps": 1e-6,
+        "rope_theta": 1e4, "tie_word_embeddings": False, "max_position_embeddings": 64}).plan())
+    model.bind({n: torch.zeros(s.shape) for n, s in model.parameters().items()}, torch.float32)
+    return model
+
+
+def facts_of(layer):
+    from socrates_b200.kernels.layer_calls import layer_facts
+    facts, tensors = [], []
+    return (facts, tensors) if layer_facts(layer, facts, tensors) else None
+
+
+def test_layers_of_equal_specs_are_alike():
+    a, b = (facts_of(layer) for layer in qwen3().layers[:2])
+    assert a[0] == b[0] and len(a[1]) == len(b[1]) == 9
+    layer = qwen3().layers[0]
+    assert {t.data_ptr() for t in layer.streamed_weights()} <= {t.data_ptr() for t in facts_of(layer)[1]}
+
+
+@pytest.mark.parametrize("change", [
+    lambda l: setattr(l.mixer, "window", 8), lambda l: setattr(l.mixer, "scale", 0.5),
+    lambda l: setattr(l.mixer, "qk_norm_eps", 1e-3), lambda l: setattr(l.mixer, "q_gain", None),
+    lambda l: setattr(l.norms[1], "eps", 1e-3), lambda l: setattr(l.feed_forward, "act", "gelu_tanh"),
+    lambda l: setattr(l.mixer.position, "magnitude", 1.5)])
+def test_a_layer_that_was_changed_is_like_no_other(change):
+    first, second = qwen3().layers[:2]
+    change(second)
+    assert facts_of(second)[0] != facts_of(first)[0]
+
+
+@pytest.mark.parametrize("pick,method", [
+    (lambda l: l, "forward"), (lambda l: l.mixer, "forward"), (lambda l: l.feed_forward, "forward"),
+    (lambda l: l.norms[0], "apply"), (lambda l: l.mixer.position, "tables"), (lambda l: l.mixer.o, "__call__")])
+@pytest.mark.parametrize("where", ["instance", "class"])
+def test_a_layer_with_a_wrapped_method_runs_by_itself(pick, method, where, monkeypatch):
+    layer = qwen3().layers[1]
+    part = pick(layer)
+    plain = getattr(type(part), method)
+    if where == "class":
+        monkeypatch.setattr(type(part), method, lambda self, *a: plain(self, *a))
+    else:
+        setattr(part, method, lambda *a: plain(part, *a))
+    assert facts_of(layer) is None
+
+
+def test_other_parts_run_by_themselves():
+    """A subclass, and a position encoding that says nothing of what its tables are."""
+    from socrates_b200.parts.attention import GQAAttention
+    from socrates_b200.parts.base import Part
+
+    class Other(GQAAttention):
+        pass
+
+    class Fresh(Part):
+        def tables(self, device):
+            return torch.zeros(8), 16
+
+    first, second = qwen3().layers[:2]
+    first.mixer.__class__ = Other
+    second.mixer.position = Fresh(None, "")
+    assert facts_of(first) is None and facts_of(second) is None
