@@ -121,7 +121,7 @@ class Model:
         is to run as any layer.  For steps that launch their kernels from here (a recorded graph needs none of this): a
         prompt portion of 187 tokens through 18 layers of the 4B shape took the host 2.9 ms in single launches, longer
         than the GPU.  What makes layers alike is looked at in every step: every class, function and constant in them, the
-        shape, type and alignment of every tensor, what the product after each is, the pages' table and what waits
+        device, shape, type and alignment of every tensor, what the product after each is, the pages' table and what waits
         on the stream."""
         layer = self.layers[self.plan.order[i].layer]
         waits = stream.pending
@@ -141,7 +141,9 @@ class Model:
             if nxt is not None and not after[-1]:
                 tensors.append(nxt)
         tensors.extend(view.pools())
-        table = view.block_table()
+        table, device = view.block_table(), waits.partial.device
+        if any([t.device != device for t in tensors]):
+            return False                                # refused, or brought over, by the layer itself
         key = (tuple(facts), tuple(after), table.data_ptr(), table.shape, waits.partial.data_ptr(), waits.partial.shape,
                tuple([(t.shape, t.dtype, t.is_contiguous(), t.data_ptr() & 127) for t in tensors]))
         addresses = [t.data_ptr() for t in tensors]

@@ -106,3 +106,29 @@ def test_other_parts_run_by_themselves():
     first.mixer.__class__ = Other
     second.mixer.position = Fresh(None, "")
     assert facts_of(first) is None and facts_of(second) is None
+
+
+def test_a_layer_with_a_tensor_elsewhere_is_left_to_the_entry_points_checks(monkeypatch):
+    from socrates_b200.engine.model import Recording
+    from socrates_b200.kernels.layer_calls import _REPLAYABLE
+    from socrates_b200.parts.base import Branch, ResidualStream
+    from socrates_b200.parts.block import PreNormBlock
+    seen, table = [], torch.zeros(1, 1)
+
+    def forward(self, ctx, stream, view):
+        seen.append("own")
+    known = _REPLAYABLE[PreNormBlock]
+    monkeypatch.setattr(PreNormBlock, "forward", forward)
+    monkeypatch.setitem(_REPLAYABLE, PreNormBlock, (known[0], forward, *known[2:]))
+    monkeypatch.setattr(Recording, "__enter__", lambda self: self)
+    monkeypatch.setattr(Recording, "__exit__", lambda self, *a: setattr(self, "words", []))
+    monkeypatch.setattr(Recording, "run", lambda self, addresses: seen.append("run"))
+    view = type("View", (), {"pools": lambda self: (torch.zeros(1), torch.zeros(1)), "block_table": lambda self: table})()
+    model, stream, recordings = qwen3(6), ResidualStream(torch.zeros(4, 32)), {}
+    stream.pending = waits = Branch(torch.zeros(1, 4, 32))
+    model.layers[2].mixer.o.weight = model.layers[2].mixer.o.weight.to("meta")
+    for i in range(1, 4):
+        stream.pending = waits
+        if not model._like_another(step(torch.float32, host_batch=[]), stream, view, i, recordings):
+            seen.append("alone")
+    assert seen[0] == "own" and seen[1] == "alone" and seen[2] in ("own", "run")
