@@ -52,7 +52,9 @@ constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;
 // TMEM columns of one block (256 allocated).  S/P buffer b occupies 64 columns at 64*b:
 // first the float32 scores of a tile, then (written over them by the softmax) the weights:
 // the high bfloat16 terms in its columns 0..31 (two keys per column), the low terms in 32..63.
+// MAPPED 3 has one S/P buffer (see the kernel): scores in columns 0..63, three terms of the weights in 0..95.
 constexpr int COL_SP = 0;
+template <int MAPPED> __device__ __forceinline__ constexpr int col_sp(int b) { return MAPPED == 3 ? COL_SP : COL_SP + 64 * b; }
 constexpr int COL_O = 128;           // D columns: the output accumulator, float32
 constexpr float RESCALE_LOG2 = 8.0f; // a row's reference maximum moves when its maximum grew by 2^8
 
@@ -196,6 +198,23 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity));
 }
 
+// tanh without a branch, so that a row's 64 lie side by side in the pipelines (tanhf takes one of two paths: 312 us a launch
+// of the size below with it, 134 with this): below 5/8 the quotient z (945 + 105 z^2 + z^4) / (945 + 420 z^2 + 15 z^4) that Lambert's
+// continued fraction z / (1 + z^2 / (3 + z^2 / (5 + ...))) gives when it is cut after 9 (off by less than 1e-9 of the value
+// there), above it (e^{2z} - 1) / (e^{2z} + 1); one reciprocal for both.  NaN stays NaN.
+__device__ __forceinline__ float tanh_select(float z) {
+    float a = fabsf(z);
+    a = a > 15.0f ? 15.0f : a;                              // 1 in float32 from 9.02 on
+    const float z2 = z * z;
+    const bool small = a < 0.625f;
+    const float e = ex2_approx(a * (2.0f * LOG2E));
+    const float num = small ? z * fmaf(z2, z2 + 105.0f, 945.0f) : copysignf(e - 1.0f, z);
+    const float den = small ? fmaf(z2, fmaf(z2, 15.0f, 420.0f), 945.0f) : e + 1.0f;
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(den));
+    return num * r;
+}
+
 // four softmax warps, the warp that issues the score products, the copy-issuing warp, the warp
 // that issues the P.V products
 constexpr int THREADS = ROWS + 96;
@@ -205,10 +224,17 @@ constexpr int THREADS = ROWS + 96;
 // MAPPED 2: the same with a cap of at most BOUND_LOG2 in units of log2.  A row's largest score then lies between minus and
 // plus the cap (the query's own position costs no slope), so 2^score itself is a weight that float32 holds with its sums:
 // no running maximum, no rescaling, and every score becomes its weight on its own.
-// MAPPED 3: as 1, and a learned bias by distance joins the score (`dist_bias`, a row per query head): a thread owns a row of
-// scores, so its 64 biases of a tile are neighbours in its head's table, read through L1.  Capped scores with such a bias
-// ran on the CUDA cores before (attention_bias.cu): 1,500 tokens, 16 query and 4 KV heads of 128, a window of 1,024:
-// 912 us a launch there, 89 us here.
+// MAPPED 3: a learned bias by distance joins the score (`dist_bias`, a row per query head): a thread owns a row of scores, so
+// its 64 biases of a tile are neighbours in its head's table, read through L1.  Such layers ran on the CUDA cores before
+// (attention_bias.cu) with scores, weights and sums in float32, and all of these bits are kept: scores stay in natural units,
+// tanh, exp and the gate are float32-accurate (tanh_select, expf), and a weight goes into the product as THREE bfloat16
+// terms, whose sum is the float32 weight itself (8 bits of its 24 each; the values are bfloat16 anyway).  Three terms of 64
+// keys are 96 columns: beside 128 of O there is room for one S/P buffer, so a tile's scores are issued once the product
+// before is done, and the SM's second block fills the gap.
+// 1,500 tokens, 16 query and 4 KV heads of 128, a window of 1,024, cap 30: 900 us a launch on the CUDA cores, 134 here (90
+// with two-term weights and hardware approximations, which lost bits).  Off from float64 before the result is rounded to
+// bfloat16 (which takes 1.7e-3): 3.2e-7 on the CUDA cores, 7.6e-7 here (the tensor core's float32 sums), 2.0e-6 with two
+// terms; after it the three agree to 1e-6 of their error.
 constexpr float BOUND_LOG2 = 80.0f;
 
 template <int D, int MAPPED>
@@ -382,7 +408,9 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_k, const __g
                 // so PV(i-2) must have COMPLETED before its weights are overwritten.  v_free[b]
                 // completes once per product on buffer b, and the next one cannot come before the
                 // scores issued here: the wait is never two phases behind.
-                if (i >= 2 && !mbar_wait_warp(smem_u32(&v_free[b]), ((i - 2) >> 1) & 1)) {
+                // With one S/P buffer (MAPPED 3) the same holds for PV(i-1).
+                constexpr int BACK = MAPPED == 3 ? 1 : 2;
+                if (i >= BACK && !mbar_wait_warp(smem_u32(&v_free[(i - BACK) & 1]), ((i - BACK) >> 1) & 1)) {
                     atomicExch(status, 13); atomicExch(&abort_flag, 1); break;
                 }
                 if (__any_sync(0xffffffffu, *((volatile int*)&abort_flag))) break;
@@ -393,7 +421,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_k, const __g
                         // the start address sits in the low bits of a descriptor in units of 16 bytes
                         const uint32_t pq = ((kk >> 2) * PANEL_Q + (kk & 3) * 32) >> 4;
                         const uint32_t pk = (b * kv_bytes<D>() + (kk >> 2) * PANEL_KV + (kk & 3) * 32) >> 4;
-                        mma_ss(tmem_u + COL_SP + 64 * b, dq + pq, dk + pk, idesc_qk, kk > 0 ? 1u : 0u);
+                        mma_ss(tmem_u + col_sp<MAPPED>(b), dq + pq, dk + pk, idesc_qk, kk > 0 ? 1u : 0u);
                     }
                     tc_commit(smem_u32(&s_full[b]));
                 }
@@ -414,7 +442,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_k, const __g
                 if (__any_sync(0xffffffffu, *((volatile int*)&abort_flag))) break;
                 tc_fence_after();
                 if (elect_one()) {
-                    const uint32_t pbase = tmem_u + COL_SP + 64 * b;
+                    const uint32_t pbase = tmem_u + col_sp<MAPPED>(b);
 #pragma unroll
                     for (int j = 0; j < KTILE / 16; ++j)
                         mma_ts(tmem_u + COL_O, pbase + j * 8, dv + ((b * kv_bytes<D>() + j * 2048) >> 4), idesc_pv,
@@ -422,6 +450,11 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_k, const __g
 #pragma unroll
                     for (int j = 0; j < KTILE / 16; ++j)
                         mma_ts(tmem_u + COL_O, pbase + 32 + j * 8, dv + ((b * kv_bytes<D>() + j * 2048) >> 4), idesc_pv, 1u);
+                    if constexpr (MAPPED == 3) {
+#pragma unroll
+                        for (int j = 0; j < KTILE / 16; ++j)
+                            mma_ts(tmem_u + COL_O, pbase + 64 + j * 8, dv + ((b * kv_bytes<D>() + j * 2048) >> 4), idesc_pv, 1u);
+                    }
                     tc_commit(smem_u32(&pv_full));
                     tc_commit(smem_u32(&v_free[b]));        // V buffer b and S/P buffer b may be reused
                 }
@@ -436,8 +469,10 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_k, const __g
         const int qpos = tok < n_tok ? first_pos + tok : -1;   // rows past the tile see no key
         const int qlo = qpos >= 0 ? first_visible(qpos, window, map.chunk) : 0;
         RowScores row_scores;
-        if constexpr (MAPPED != 0) row_scores.set(map, scale_log2, kh * G + g);
+        if constexpr (MAPPED == 1 || MAPPED == 2) row_scores.set(map, scale_log2, kh * G + g);
         const float* bias_row = MAPPED == 3 ? dist_bias + (size_t)(kh * G + g) * bias_len : nullptr;
+        const float in_cap = MAPPED == 3 && map.cap > 0.f ? scale_log2 / map.cap : 0.f;
+        const float slope = MAPPED == 3 && map.slopes != nullptr ? map.slopes[kh * G + g] : 0.f;
         const float per_unit = MAPPED != 0 ? 1.0f : scale_log2;     // from the scores below to exponents of 2
         const uint32_t lane_base = tmem + (static_cast<uint32_t>(warp * 32) << 16);
         bool ok = true;
@@ -453,29 +488,31 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_k, const __g
             float s[64];
             {
                 uint32_t raw[32];
-                tmem_ld32(lane_base + COL_SP + 64 * b, raw);
+                tmem_ld32(lane_base + col_sp<MAPPED>(b), raw);
                 tmem_ld_wait();
 #pragma unroll
                 for (int j = 0; j < 32; ++j) s[j] = __uint_as_float(raw[j]);
-                tmem_ld32(lane_base + COL_SP + 64 * b + 32, raw);
+                tmem_ld32(lane_base + col_sp<MAPPED>(b) + 32, raw);
                 tmem_ld_wait();
 #pragma unroll
                 for (int j = 0; j < 32; ++j) s[32 + j] = __uint_as_float(raw[j]);
             }
-            if constexpr (MAPPED != 0) {
-                row_scores.from((float)(tile_start - qpos));
-                if constexpr (MAPPED == 3) {
-                    const int ahead = qpos - tile_start;     // key j of the tile is ahead - j away
-                    if (row_scores.capped) {
+            if constexpr (MAPPED == 3) {
+                const int ahead = qpos - tile_start;         // key j of the tile is ahead - j away
+                auto bias = [&](int j) { return __ldg(bias_row + min(max(ahead - j, 0), bias_len - 1)); };
+                if (map.cap > 0.f) {
 #pragma unroll
-                        for (int j = 0; j < 64; ++j)
-                            s[j] = fmaf(__ldg(bias_row + min(max(ahead - j, 0), bias_len - 1)), LOG2E, row_scores.with_cap(s[j], (float)j));
-                    } else {
+                    for (int j = 0; j < 64; ++j) s[j] = fmaf(map.cap, tanh_select(s[j] * in_cap), bias(j));
+                } else {
 #pragma unroll
-                        for (int j = 0; j < 64; ++j)
-                            s[j] = fmaf(__ldg(bias_row + min(max(ahead - j, 0), bias_len - 1)), LOG2E, row_scores.plain(s[j], (float)j));
-                    }
+                    for (int j = 0; j < 64; ++j) s[j] = fmaf(s[j], scale_log2, bias(j));       // the plain scale
                 }
+                if (slope != 0.f) {
+#pragma unroll
+                    for (int j = 0; j < 64; ++j) s[j] -= slope * (float)(ahead - j);
+                }
+            } else if constexpr (MAPPED != 0) {
+                row_scores.from((float)(tile_start - qpos));
                 if (MAPPED == 1 && row_scores.capped) {
 #pragma unroll
                     for (int j = 0; j < 64; ++j) s[j] = row_scores.with_cap(s[j], (float)j);
@@ -488,13 +525,13 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_k, const __g
             // rows past the tile (qpos = -1) are masked by the same test
             const bool masked = i < keep_tiles ? (tile_start + KTILE > kf || n_tok < TQ)
                                                : (tile_start + KTILE - 1 > first_pos || tile_start < last_qlo || n_tok < TQ);
-            // weights (of key j of the tile: weight(j)), their sum, and their two terms over the scores of this very row,
-            // all 64 of which were read into registers above
+            // weights (of key j of the tile: weight(j)), their sum, and their two or three terms over the scores of this very
+            // row, all 64 of which were read into registers above
             auto write_weights = [&](auto weight) {
                 float l4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int c = 0; c < KTILE; c += 32) {
-                    uint32_t ph[16], pl[16];
+                    uint32_t ph[16], pl[16], pr[16];
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         const float p0 = weight(c + 2 * j);
@@ -502,10 +539,15 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_k, const __g
                         l4[j & 3] += p0 + p1;
                         const uint32_t h = pack_bf16(p0, p1);
                         ph[j] = h;
-                        pl[j] = pack_bf16(p0 - __uint_as_float(h << 16), p1 - __uint_as_float(h & 0xffff0000u));
+                        const float r0 = p0 - __uint_as_float(h << 16), r1 = p1 - __uint_as_float(h & 0xffff0000u);
+                        const uint32_t l = pack_bf16(r0, r1);
+                        pl[j] = l;
+                        if constexpr (MAPPED == 3)
+                            pr[j] = pack_bf16(r0 - __uint_as_float(l << 16), r1 - __uint_as_float(l & 0xffff0000u));
                     }
-                    tmem_st16(lane_base + COL_SP + 64 * b + (c >> 1), ph);
-                    tmem_st16(lane_base + COL_SP + 64 * b + 32 + (c >> 1), pl);
+                    tmem_st16(lane_base + col_sp<MAPPED>(b) + (c >> 1), ph);
+                    tmem_st16(lane_base + col_sp<MAPPED>(b) + 32 + (c >> 1), pl);
+                    if constexpr (MAPPED == 3) tmem_st16(lane_base + col_sp<MAPPED>(b) + 64 + (c >> 1), pr);
                 }
                 l_run += (l4[0] + l4[1]) + (l4[2] + l4[3]);
             };
@@ -536,11 +578,11 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_k, const __g
             }
             const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
             // lazy rescale: move the reference maximum only when the row maximum outgrew it
-            const bool grow = mx > -INFINITY && (m_ref == -INFINITY || (mx - m_ref) * per_unit > RESCALE_LOG2);
+            const bool grow = mx > -INFINITY && (m_ref == -INFINITY || (mx - m_ref) * (MAPPED == 3 ? LOG2E : per_unit) > RESCALE_LOG2);
             if (__any_sync(0xffffffffu, grow)) {
                 float alpha = 1.0f;
                 if (grow) {
-                    alpha = m_ref == -INFINITY ? 0.f : exp2f((m_ref - mx) * per_unit);
+                    alpha = m_ref == -INFINITY ? 0.f : (MAPPED == 3 ? expf(m_ref - mx) : exp2f((m_ref - mx) * per_unit));
                     m_ref = mx;
                     l_run *= alpha;
                 }
@@ -568,7 +610,8 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_k, const __g
             }
             // p = 2^((s - m) * scale) as one multiply-add and one ex2; masked scores are -inf -> 0
             const float neg_m = m_ref == -INFINITY ? 0.f : -m_ref * per_unit;
-            write_weights([&](int j) { return ex2_approx(fmaf(s[j], per_unit, neg_m)); });
+            if constexpr (MAPPED == 3) write_weights([&](int j) { return expf(s[j] + neg_m); });
+            else write_weights([&](int j) { return ex2_approx(fmaf(s[j], per_unit, neg_m)); });
             }
             tmem_st_wait();
             // slots of this tile outside [lo, hi): zero their V rows (thread j < 64 owns key j)
@@ -634,7 +677,10 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_k, const __g
                 const bf16* grow_ptr = gate ? gate + (size_t)(t0 + (tok < n_tok ? tok : 0)) * gate_stride +
                                                   (gate_per_dim ? (size_t)(kh * G + g) * D : (size_t)(kh * G + g)) : nullptr;
                 float head_gate = 1.0f;
-                if (gate && !gate_per_dim && tok < n_tok) head_gate = 1.0f / (1.0f + __expf(-__bfloat162float(grow_ptr[0])));
+                if (gate && !gate_per_dim && tok < n_tok) {
+                    const float z = -__bfloat162float(grow_ptr[0]);
+                    head_gate = 1.0f / (1.0f + (MAPPED == 3 ? expf(z) : __expf(z)));
+                }
 #pragma unroll
                 for (int c = 0; c < D; c += 32) {
                     uint32_t ov[32];
@@ -705,7 +751,7 @@ int launch(const CUtensorMap& mk, const CUtensorMap& mv, void* out, const void* 
     sb::launch(kernel, grid, dim3(THREADS), smem_bytes<D>() + table_width * 4, stream, mk, mv, (bf16*)out,
                (const bf16*)q, block_table, table_width, seq_starts, seq_rows, seq_first_pos, R, Hq, Hkv, BS, window,
                MAPPED != 0 ? scale : scale * LOG2E, status, (const bf16*)gate, gate_stride, gate_per_dim, has_sink,
-               has_sink ? (MAPPED != 0 ? sink * LOG2E : sink / scale) : 0.f, keep_first, out_f32, skip_single, map,
+               has_sink ? (MAPPED == 3 ? sink : MAPPED != 0 ? sink * LOG2E : sink / scale) : 0.f, keep_first, out_f32, skip_single, map,
                dist_bias, bias_len);
     return 0;
 }

@@ -12,7 +12,9 @@ with B the rows of the table `rel` [B, heads] (read from the tensor's shape) and
 Keys have `key_dim` dims and values `value_dim`; the convolved k and v go to the row's pages
 (a windowed page group: pages behind the window are given back), the last K-1 projected values
 of every sequence live in a state slot, and the bucket function is turned into a table by
-distance once, on the host, in double precision.  The four projections are one matrix product.
+distance once, on the host, in double precision.  The four projections are one matrix product.  Scores, softmax weights and sums
+are float32 in every kernel that serves this part (the tensor-core kernel for prompt portions carries a weight as three
+bfloat16 terms).
 Tensors: `<name>q`, `q.b`, `q.conv`, the same for k and v, `rel`, `g`, `o`.
 """
 
