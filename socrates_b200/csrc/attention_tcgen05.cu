@@ -170,6 +170,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 
 template <int D> constexpr int q_bytes() { return ROWS * D * 2; }
 template <int D> constexpr int kv_bytes() { return KTILE * D * 2; }          // one of K or V, one buffer
+constexpr int MAX_TABLE = 4096;      // columns of the block table (a tile's share of a row is held in shared memory)
 template <int D> constexpr int smem_bytes() { return q_bytes<D>() + 4 * kv_bytes<D>() + 1024; }
 
 // ----------------------------------------------------------------------------- the kernel
@@ -742,7 +743,7 @@ int launch(const CUtensorMap& mk, const CUtensorMap& mv, void* out, const void* 
     bool& configured = once_per_device.flag();
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             smem_bytes<D>() + 4096 * 4);
+                                             smem_bytes<D>() + MAX_TABLE * 4);
         if (e != cudaSuccess) { sb_set_error("attention_tcgen05: %s", cudaGetErrorString(e)); return (int)e; }
         configured = true;
     }
@@ -764,6 +765,11 @@ extern "C" int sb_attention_tcgen05_supports(int Hq, int Hkv, int D, int page_si
     if (!(D == 64 || D == 128)) return 0;
     if (!(page_size == 16 || page_size == 32 || page_size == 64)) return 0;
     return Hq / Hkv <= ROWS;       // a group that does not divide 128 leaves the last rows of a tile unused
+}
+
+// 1 if it takes pools of so many pages and block tables of this width, else 0.
+extern "C" int sb_attention_tcgen05_pages_supports(int num_pages, int Hkv, int page_size, int table_width) {
+    return num_pages > 0 && (long long)num_pages * Hkv * page_size < (1ll << 31) && table_width > 0 && table_width <= MAX_TABLE;
 }
 
 // Arguments as sb_attention_prefill_mma, plus `num_pages` (pages of the pools, the null
@@ -792,10 +798,10 @@ extern "C" int sb_attention_prefill_tcgen05(void* out, const void* q, const void
         gate_per_dim = 2;                                  // 16-byte loads of the gate
     SB_REQUIRE(sb_attention_tcgen05_supports(Hq, Hkv, D, page_size),
                "attention_tcgen05: Hq=%d Hkv=%d head_dim=%d page_size=%d is not supported", Hq, Hkv, D, page_size);
-    SB_REQUIRE(R > 0 && N > 0 && window >= 0 && table_width > 0 && table_width <= 4096 && num_pages > 0,
-               "attention_tcgen05: bad sizes R=%d N=%d table_width=%d", R, N, table_width);
+    SB_REQUIRE(R > 0 && N > 0 && window >= 0, "attention_tcgen05: bad sizes R=%d N=%d window=%d", R, N, window);
+    SB_REQUIRE(sb_attention_tcgen05_pages_supports(num_pages, Hkv, page_size, table_width),
+               "attention_tcgen05: %d pages, table_width=%d (at most %d)", num_pages, table_width, MAX_TABLE);
     SB_REQUIRE(status != nullptr, "attention_tcgen05: status is required");
-    SB_REQUIRE((long long)num_pages * Hkv * page_size < (1ll << 31), "attention_tcgen05: pool too large");
     CUtensorMap mk, mv;
     const int rows = num_pages * Hkv * page_size;
     if (!sb::get_map(&mk, k_pool, rows, D, page_size) || !sb::get_map(&mv, v_pool, rows, D, page_size)) {

@@ -527,6 +527,12 @@ def attention_tcgen05_supports(num_heads: int, num_kv_heads: int, head_dim: int,
     return bool(library().sb_attention_tcgen05_supports(num_heads, num_kv_heads, head_dim, page_size))
 
 
+def attention_tcgen05_pages_supports(k_pool: torch.Tensor, block_table: torch.Tensor) -> bool:
+    """Whether it takes pools and block tables of this size (rows of at most 4,096 pages)."""
+    pages, Hkv, BS, _ = k_pool.shape
+    return bool(library().sb_attention_tcgen05_pages_supports(pages, Hkv, BS, block_table.shape[1]))
+
+
 def attention_prefill_tcgen05(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
                               block_table: torch.Tensor, seq_starts: torch.Tensor, seq_rows: torch.Tensor,
                               seq_first_pos: torch.Tensor, num_heads: int, scale: float, status: torch.Tensor,

@@ -128,12 +128,13 @@ class WindowBiasAttention(Part):
         gate = qkvg[:, self.C:self.C + self.H]
         portions = not ctx.all_decode and N >= 4 * ctx.num_seqs
         if (portions and ctx.dtype == torch.bfloat16 and self.dk == self.dv and ctx.status is not None
-                and ops.attention_tcgen05_supports(self.H, self.G, self.dk, k_pool.shape[2])):
+                and ops.attention_tcgen05_supports(self.H, self.G, self.dk, k_pool.shape[2])
+                and ops.attention_tcgen05_pages_supports(k_pool, table)):
             ops.attention_prefill_tcgen05(attn, q, k_pool, v_pool, table, ctx.seq_starts, ctx.seq_rows, ctx.seq_first_pos,
                                           self.H, self.scale, ctx.status, self.window or 0, gate=gate,
-                                          softcap=self.softcap, dist_bias=self.dist_bias)
+                                          softcap=max(self.softcap, 0.0), dist_bias=self.dist_bias)
             return Branch(self.o(ctx, attn, self.out_buffer, out="partial"))
-        if (portions and ops.attention_bias_tile_supports(self.H, self.G, self.dk, self.dv, ctx.dtype)):
+        if portions and ops.attention_bias_tile_supports(self.H, self.G, self.dk, self.dv, ctx.dtype):
             # prompt portions: a tile of a request's consecutive tokens per block shares the keys it reads
             ops.attention_bias_tile(attn, q, k_pool, v_pool, table, ctx.seq_starts, ctx.seq_rows, ctx.seq_first_pos,
                                     self.H, self.scale, self.window or 0, self.softcap, self.dist_bias, gate=gate)

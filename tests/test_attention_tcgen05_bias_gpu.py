@@ -104,3 +104,22 @@ def test_bias_of_the_lowest_value(ops):
     ops.attention_bias_tile(before, q, k_pool, v_pool, table, *seq, Hq, D ** -0.5, 0, 5.0, bias, gate=gate)
     # one rounding to bfloat16 apart (2^-8 of a value where it falls on the other side)
     assert int(status) == 0 and bool(before.isfinite().all()) and torch.allclose(out.float(), before.float(), rtol=2.0 ** -7, atol=1e-5)
+
+
+def test_a_table_wider_than_the_tile_kernel_takes(ops):
+    """Short rows in a cache of very long ones: the tile kernel refuses the table, the CUDA-core kernel serves it."""
+    from socrates_b200.kernels.library import KernelError
+    Hq, Hkv, D = 4, 2, 64
+    k_pool, v_pool, table = paged_case([70], 16, Hkv, D, BF, seed=6)
+    wide = torch.zeros(1, 4097, dtype=torch.int32, device=DEV)
+    wide[:, :table.shape[1]] = table
+    q, gate, bias = rand(70, Hq * D, dtype=BF, seed=7), rand(70, Hq, dtype=BF, seed=8), rand(Hq, 40, dtype=torch.float32, seed=9)
+    seq, status = (as_int([0, 70]), as_int([0]), as_int([0])), torch.zeros(1, dtype=torch.int32, device=DEV)
+    assert not ops.attention_tcgen05_pages_supports(k_pool, wide)
+    assert ops.attention_tcgen05_pages_supports(k_pool, wide[:, :4096])
+    out, narrow = torch.empty_like(q), torch.empty_like(q)
+    with pytest.raises(KernelError):
+        ops.attention_prefill_tcgen05(out, q, k_pool, v_pool, wide, *seq, Hq, D ** -0.5, status, 0, gate=gate, dist_bias=bias)
+    ops.attention_bias_tile(out, q, k_pool, v_pool, wide, *seq, Hq, D ** -0.5, 0, 30.0, bias, gate=gate)
+    ops.attention_bias_tile(narrow, q, k_pool, v_pool, table, *seq, Hq, D ** -0.5, 0, 30.0, bias, gate=gate)
+    assert torch.equal(out, narrow)

@@ -132,3 +132,29 @@ def test_a_layer_with_a_tensor_elsewhere_is_left_to_the_entry_points_checks(monk
         if not model._like_another(step(torch.float32, host_batch=[]), stream, view, i, recordings):
             seen.append("alone")
     assert seen[0] == "own" and seen[1] == "alone" and seen[2] in ("own", "run")
+
+
+# ---------------------------------------------------------------------- kernels by the sizes of the cache
+@pytest.mark.parametrize("pages,width,kernel", [
+    (600, 4096, "attention_prefill_tcgen05"), (600, 4097, "attention_bias_tile"),     # 65,536 tokens in pages of 16
+    (2 ** 25, 64, "attention_bias_tile")])                                            # 2^31 key rows in a pool
+def test_windowed_attention_with_a_bias_takes_caches_of_any_size(pages, width, kernel, monkeypatch):
+    from socrates_b200.config.plan import PartSpec
+    from socrates_b200.parts import window_attention
+    from socrates_b200.parts.window_attention import WindowBiasAttention
+    part = WindowBiasAttention(PartSpec("window_bias_attention", dict(
+        hidden_size=32, num_heads=4, num_kv_heads=4, key_dim=64, value_dim=64, scale=0.1, window=None, bias_far=16.0,
+        softcap=-1.0)), "")
+    ran = []
+    for name in ("attention_prefill_tcgen05", "attention_bias_tile", "attention_bias"):
+        monkeypatch.setattr(window_attention.ops, name, lambda *a, name=name, softcap=0.0, **k: ran.append((name, softcap)))
+    monkeypatch.setattr(window_attention.ops, "short_conv", lambda *a: None)
+    part.qkvg = lambda ctx, x, name: torch.zeros(x.shape[0], part.C + part.H)
+    part.o = lambda ctx, x, name, out: torch.zeros(1, x.shape[0], 32)
+    ctx = step(status=torch.zeros(1, dtype=torch.int32))
+    ctx.all_decode, ctx.num_tokens = False, 40
+    pool = torch.empty(pages, 4, 16, 64, device="meta", dtype=torch.bfloat16)
+    cache = type("View", (), {"pools": lambda self: (pool, pool), "block_table": lambda self: torch.empty(4, width, device="meta")})()
+    part.forward(ctx, torch.zeros(40, 32), cache)
+    assert [name for name, _ in ran] == [kernel]
+    assert kernel != "attention_prefill_tcgen05" or ran[0][1] >= 0    # a cap below zero was, and is, no cap
