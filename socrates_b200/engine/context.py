@@ -182,25 +182,26 @@ class StepContext:
         twice and 256-wide ones leave half of the SMs idle), else 0.
 
         As many parts as there are places (two blocks an SM up to 128 rows, one beyond), at least four K blocks each; it
-        takes three parts to beat the other kernels.  Measured (us, before / so): 187 rows: 2,560 x 4,096 16.8 / 11.4,
-        2,560 x 9,728 26.1 / 16.7, 6,144 x 2,560 16.8 / 13.3, 5,120 x 25,600 70.8 / 59.5, 4,096 x 12,288 30.5 / 28.7; 72
-        rows: 13.0 / 8.1, 21.7 / 12.9, 12.1 / 9.7, 56.0 / 54.4, 27.0 / 22.6.  256 columns are a heavier tile: there only
-        where nine tenths of the SMs get a block (2,560 x 9,728 26.5 / 19.3, but 4,096 x 12,288 31.8 / 33.8).
-        A short product that narrows follows attention, whose blocks hold a third of the SMs: with one block an SM its
-        blocks should all find room beside them, so that their first weights are there when attention ends (4,096 x 4,096
-        in 128 blocks ended 27 us after it in the 8B step, the kernel before in 13), and there must be four parts of it."""
+        takes three parts to beat the other kernels.  Measured (us, the other kernels / so, in a graph over weights that
+        no cache holds): 187 rows: 2,560 x 4,096 17.3 / 11.6, 2,560 x 9,728 26.4 / 17.2, 6,144 x 2,560 17.0 / 13.5,
+        5,120 x 25,600 70.2 / 59.3, 4,096 x 12,288 30.5 / 28.7; 72 rows: 13.0 / 8.9, 22.0 / 12.5, 12.8 / 9.4, 55.0 / 47.1,
+        27.1 / 22.2.  256 columns are a heavier tile: there only where nine tenths of the SMs get a block (250 rows: 2,560
+        x 9,728 26.8 / 19.8, but 4,096 x 12,288 31.6 / 33.6).
+        A short product that narrows (N <= K <= 8,192: what follows attention) starts beside attention's blocks, which
+        hold a third of the SMs, and with one block an SM most of what it gains alone is lost there: what counts is the
+        step.  Measured in steps of one prompt (us a step, other kernels / so), 2,560 x 4,096 in seven parts (18 layers of
+        4B): 130 rows 2,518 / 2,422, 160 2,491 / 2,423, 187 2,536 / 2,538, 200 2,757 / 2,775 (in five parts 50 more each);
+        4,096 x 4,096 in four (12 layers of 8B): 130 2,301 / 2,322, 187 2,372 / 2,457; 5,120 x 8,192 in three (4 layers of
+        32B): 160 1,486 / 1,521, 187 equal, 250 1,627 / 1,676.  So there with five parts and more, up to 192 rows."""
         if not 64 < M <= 256 or not self.uses_tensor_cores(x_dtype, w):
             return 0
         N, K = w.shape
         tiles = -(-N // 128)
         parts = min((2 if M <= 128 else 1) * self.num_sms // tiles, -(-K // 64) // 4, 14)
-        if M > 192 and 10 * tiles * parts < 9 * self.num_sms:
-            return 0
-        if M > 128 and N <= K < 8192:
-            parts = min(parts, 7 * self.num_sms // 10 // tiles)
-            if parts < 4:
+        if N <= K <= 8192 and M > 128:
+            if parts < 5 or M > 192:
                 return 0
-        if parts < 3:
+        elif parts < 3 or (M > 192 and 10 * tiles * parts < 9 * self.num_sms):
             return 0
         return ops.gemm_tcgen05_splits(K, parts)
 

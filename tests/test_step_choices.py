@@ -158,3 +158,16 @@ def test_windowed_attention_with_a_bias_takes_caches_of_any_size(pages, width, k
     part.forward(ctx, torch.zeros(40, 32), cache)
     assert [name for name, _ in ran] == [kernel]
     assert kernel != "attention_prefill_tcgen05" or ran[0][1] >= 0    # a cap below zero was, and is, no cap
+
+
+@pytest.mark.parametrize("M,N,K,parts", [
+    (64, 2560, 4096, 0), (65, 2560, 4096, 13), (128, 2560, 4096, 13), (129, 2560, 4096, 7), (192, 2560, 4096, 7),
+    (193, 2560, 4096, 0), (250, 2560, 4096, 0),                            # follows attention: not in a few heavy tiles
+    (129, 4096, 4096, 0), (187, 5120, 8192, 0), (128, 4096, 4096, 8),      # ... nor in fewer than five parts
+    (187, 2560, 9728, 7), (250, 2560, 9728, 7), (187, 4096, 12288, 4),
+    (193, 4096, 12288, 0), (256, 5120, 25600, 0), (256, 6144, 2560, 3), (257, 2560, 9728, 0)])
+def test_parts_of_products_of_65_to_256_rows(M, N, K, parts):
+    """Tiles of 256 columns only where nine tenths of the SMs get a block, whatever the rule for short products is."""
+    ctx, w = step(status=torch.zeros(1, dtype=torch.int32)), torch.empty(N, K, device="meta", dtype=torch.bfloat16)
+    assert ctx.wide_splits(M, w, torch.bfloat16) == parts
+    assert parts == 0 or M <= 192 or 10 * -(-N // 128) * parts >= 9 * 148
