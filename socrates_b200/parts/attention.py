@@ -39,20 +39,25 @@ def paged_partition() -> Optional[int]:
     return n
 
 
+def partitions_in(places: int, blocks: int, most: int = 16) -> int:
+    """Key partitions of the split-key decode kernel for `blocks` (token, KV head) pairs on a GPU that holds `places` of its
+    blocks at once: as many as keep every block resident, at most `most` and at most 16."""
+    parts = max(1, min(places // max(1, blocks), most, 16))
+    # 3 and 4 partitions are clusters that do not fill the last places of every GPC: with 9 rows of 8 KV heads
+    # 4 partitions (288 of 296 places) take 26 us for 2,048 keys where 3 take 19, with 12 rows of 4,000 keys 3 take 56 us
+    # and 2 take 42; 11 rows and 3 (264 places) still fit.
+    while 3 <= parts <= 4 and blocks * parts > 0.9 * places:
+        parts -= 1
+    return parts
+
+
 def decode_partitions(ctx, num_kv_heads: int, blocks_per_sm: int, keys_per_part: int) -> int:
     """Into how many key partitions the split-key decode kernel cuts each token's keys when
     PAGED_PARTITION is "auto": as many as keep every block resident at once (one wave, no tail),
     at most 16, never less than `keys_per_part` keys of the longest possible row in a partition.
     A function of the batch width and of limits only, so that a recorded graph stays valid."""
-    most = max(1, -(-ctx.max_context // keys_per_part))
-    blocks = max(1, num_kv_heads * ctx.num_tokens)
-    parts = max(1, min((ctx.num_sms * blocks_per_sm) // blocks, most, 16))
-    # 3 and 4 partitions are clusters that do not fill the last places of every GPC: with 9 rows of 8 KV heads
-    # 4 partitions (288 of 296 places) take 26 us for 2,048 keys where 3 take 19, with 12 rows of 4,000 keys 3 take 56 us
-    # and 2 take 42; 11 rows and 3 (264 places) still fit.
-    while 3 <= parts <= 4 and blocks * parts > 0.9 * ctx.num_sms * blocks_per_sm:
-        parts -= 1
-    return parts
+    return partitions_in(ctx.num_sms * blocks_per_sm, max(1, num_kv_heads * ctx.num_tokens),
+                         max(1, -(-ctx.max_context // keys_per_part)))
 
 
 # In a step that mixes prompt portions with decoding requests the tile kernel can serve both (a decoding request is a tile
@@ -203,17 +208,20 @@ class GQAAttention(Part):
         rather than cut every row into the same number of partitions.
 
         In tiles of 64 keys, a block of the split-key kernel takes ceil(longest / partitions) and one of the other T / W;
-        a row that two shares cut costs both a merge through memory, and the launch about 5 us.  Measured (us, 32 query and
-        8 KV heads of 128, split-key / shares; in brackets the tiles that a split-key block has more): 16 rows of 4,000
-        keys (4) 45 / 50, 32 of 2,048 (4) 43 / 50, 18 of 125 to 2,000 (8) 23 / 22, 10 of 250 to 4,000 (8) 27 / 22, 24 of
-        2,048 (12) 42 / 40, 12 of 250 to 4,000 (15) 39 / 25, 19 of 2,000 (16) 39 / 34: from 8 tiles on.  More rows than shares
-        are no partitions but whole rows in a second round of blocks: 64 rows of 512 keys 28 / 31, 48 of 1,000 46 / 40, 64 of
-        2,048 87 / 89, 64 of 128 to 2,048 65 / 59, 64 of 256 to 4,096 124 / 96: from 16 tiles in the longest row on."""
+        a row that two shares cut costs both a merge through memory, and the launch about 4 us.  (A short cache may leave
+        fewer partitions than counted here; they hold 128 keys then, two tiles.)  Measured (us a launch in a graph, keys in
+        no cache, 32 query and 8 KV heads of 128, split-key / shares; `a to b`: lengths evenly spaced; in brackets the tiles
+        that a split-key block has more): 9 rows of 4,000 keys (6) 30.0 / 31.7, 12 of 2,000 (6) 24.9 / 24.5, 18 of 125 to
+        2,000 (8) 23.6 / 22.4, 32 of 4,000 (8) 81.0 / 86.7, 16 of 125 to 2,000 (9) 22.3 / 20.6, 13 of 4,000 (10) 41.9 / 41.5,
+        24 of 2,000 (11) 40.1 / 39.5, 12 of 4,000 (12) 41.8 / 38.8, 10 of 250 to 4,000 (12) 27.1 / 23.7, 19 of 2,000 (16)
+        38.9 / 33.2, 12 of 250 to 4,000 (21) 36.5 / 25.5; 16 KV heads: 6 of 4,000 (11) 41.0 / 37.5; 4: 24 of 4,000 (12) 43.1 /
+        41.1; 2: 36 of 250 to 4,000 (13) 27.7 / 25.9.  So from 8 tiles on.  More rows than shares are no partitions but whole
+        rows in a second round of blocks: 64 rows of 512 keys 27.6 / 30.2, 48 of 1,000 45.8 / 39.8, 64 of 2,048 85.8 / 88.6,
+        64 of 128 to 2,048 57.9 / 57.4, 64 of 256 to 4,096 109.4 / 97.7: from 16 tiles in the longest row on."""
         N = len(lengths)
         if N < 5 or paged_partition() is not None:          # few rows are cut into many partitions each: even anyway
             return False
-        per_sm = ops.attention_decode_mma_blocks_per_sm(self.D)
-        parts = max(1, min((num_sms * per_sm) // max(1, self.Hkv * N), 16))
+        parts = partitions_in(num_sms * ops.attention_decode_mma_blocks_per_sm(self.D), self.Hkv * N)
         shares = ops.attention_balanced_shares(self.Hq, self.Hkv, self.D, N, num_sms)
         if self.window:
             lengths = [min(n, self.window) for n in lengths]

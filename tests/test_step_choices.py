@@ -171,3 +171,22 @@ def test_parts_of_products_of_65_to_256_rows(M, N, K, parts):
     ctx, w = step(status=torch.zeros(1, dtype=torch.int32)), torch.empty(N, K, device="meta", dtype=torch.bfloat16)
     assert ctx.wide_splits(M, w, torch.bfloat16) == parts
     assert parts == 0 or M <= 192 or 10 * -(-N // 128) * parts >= 9 * 148
+
+
+@pytest.mark.parametrize("Hkv,lengths,shares", [
+    (8, [4000] * 9, False), (8, [4000] * 11, False), (8, [4000] * 12, True), (8, [2000] * 12, False),
+    (8, [4000] + [250] * 8, True), (16, [4000] * 6, True), (16, [4000] * 7, False), (4, [4000] * 18, False),
+    (4, [4000] * 24, True), (2, [4000] * 36, False), (2, [4000] * 48, True), (8, [2048] * 8, False)])
+def test_shares_are_weighed_against_the_partitions_that_the_launch_has(Hkv, lengths, shares):
+    """Counts of 3 and 4 partitions are stepped down where clusters fill the GPU badly; the rule counts with the same number."""
+    from socrates_b200.config.plan import PartSpec
+    from socrates_b200.kernels import ops
+    from socrates_b200.parts.attention import GQAAttention, decode_partitions
+    part = GQAAttention(PartSpec("gqa_attention", dict(hidden_size=64, num_heads=32, num_kv_heads=Hkv, head_dim=128,
+                                                       position=PartSpec("none", {}))), "")
+    assert part.prefers_shares(lengths, 148) == shares
+    ctx = step()
+    ctx.num_tokens = N = len(lengths)
+    NP = decode_partitions(ctx, Hkv, ops.attention_decode_mma_blocks_per_sm(128), 128)
+    longest, total = -(-max(lengths) // 64), sum(lengths) / 64 + N / 2
+    assert (-(-longest // NP) - total / ops.attention_balanced_shares(32, Hkv, 128, N, 148) >= 8) == shares
