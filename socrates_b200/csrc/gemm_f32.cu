@@ -333,9 +333,12 @@ int gemm_f32(float* C, const float* A, const float* W, int M, int N, int K, int 
         configured = true;
     }
     const int row_tiles = (M + TILE - 1) / TILE, tiles = row_tiles * ((N + TILE - 1) / TILE);
-    // Below three tiles for each of the GPU's 296 places whole tiles fill their last round badly: a tile is dealt to four
-    // blocks then.
-    if (tiles < 888)
+    int dev = 0, num_sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+    // Below three tiles for each of the GPU's places (two blocks an SM) whole tiles fill their last round badly: a tile is
+    // dealt to four blocks then.
+    if (tiles < 3 * 2 * num_sms)
         sb::launch_cluster(gemm_f32_tile_kernel<true>, dim3(tiles * GROUPS), dim3(NTHR), TILE_SMEM, stream, dim3(GROUPS), C, A, W,
                            M, N, K, row_tiles, w_older);
     else
