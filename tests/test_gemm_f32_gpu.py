@@ -32,6 +32,24 @@ def test_gemm_f32(ops, N, K):
         assert torch.equal(out, whole[:M]), M
 
 
+@pytest.mark.parametrize("N,K,rows", [(57600, 520, (65, 9, 64, 1, 8)), (14400, 1036, (256, 9, 64, 130, 1, 5))])
+def test_whole_tiles_of_many_pieces(ops, N, K, rows):
+    """Products with tiles enough for whole tiles (888 on 148 SMs) whose segments hold two to five pieces each, the last one
+    cut: the refills and the joining of segments carry the result there.  14,400 columns by 64 rows and fewer are clusters
+    of the same sums."""
+    M = rows[0]
+    a, w = rand(M, K, dtype=torch.float32, seed=1), rand(N, K, dtype=torch.float32, seed=2)
+    exact = a.double() @ w.double().T
+    bound = (K / 16 + 6) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)      # as above
+    whole = torch.full((M, N), float("nan"), device=DEV)
+    ops.gemm_simt(whole, a, w)
+    assert bool(((whole.double() - exact).abs() <= bound).all())
+    for m in rows[1:]:
+        out = torch.full((m, N), float("nan"), device=DEV)
+        ops.gemm_simt(out, a[:m].contiguous(), w)
+        assert torch.equal(out, whole[:m]), m
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 2560, 1024), (8, 2560, 1024), (70, 2560, 1024), (64, 57600, 64)])
 def test_a_matrix_that_the_kernel_before_writes(ops, M, N, K):
     """w is the result of the kernel right before this one on the stream, which lets its successor start early: nothing of
