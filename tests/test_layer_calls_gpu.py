@@ -28,7 +28,7 @@ def build(dtype, layers=6, window=None, seed=0):
                   num_blocks=400)
 
 
-def steps(engine):
+def steps(engine, after_step=lambda: None):
     """Logits of a prompt, of its second portion beside two new prompts, and of a step that mixes both kinds."""
     from socrates_b200.engine.runner import StepEntry
     g = torch.Generator().manual_seed(5)
@@ -43,6 +43,7 @@ def steps(engine):
             assert cache.reserve(row, start + n)
             entries.append(StepEntry(row, ids(n), start, [n - 1]))
         out.append(engine.runner.step(entries).logits.clone())
+        after_step()
         for row, n in portions:
             at[row] = at.get(row, 0) + n
             cache.commit(row, at[row])
@@ -57,8 +58,11 @@ def test_recorded_layers_give_the_same_bits(dtype, window, monkeypatch):
     runs = []
     run = Recording.run
     monkeypatch.setattr(Recording, "run", lambda self, a: (runs.append(1), run(self, a))[1])
-    got, launches = steps(build(dtype, window=window))
-    assert len(runs) >= 4                               # every step had layers that ran from another's calls
+    so_far = []
+    got, launches = steps(build(dtype, window=window), lambda: so_far.append(len(runs)))
+    # in every step: of six layers alike the first finds nothing pending, the second is recorded and the last is followed
+    # by another matrix; of three and three (with a window) only the fifth runs from another's calls
+    assert so_far == [n * (3 if window is None else 1) for n in (1, 2, 3, 4)]
     monkeypatch.setattr(Model, "_like_another", lambda *a: False)
     want, plain = steps(build(dtype, window=window))
     assert launches == plain
@@ -80,6 +84,48 @@ def test_a_layer_with_a_tensor_of_another_type_runs_by_itself(monkeypatch):
     monkeypatch.setattr(Model, "_like_another", lambda *a: False)
     want, plain = steps(odd())
     assert launches == plain and all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("how,kernel", [("auto", "sb_attention_decode_mma"), ("64", "sb_attention_decode_stream"),
+                                        ("shares", "sb_attention_balanced"), ("mixed", "sb_attention_balanced")])
+def test_decode_kernels_from_recorded_calls(how, kernel, monkeypatch):
+    """The first step of a width, which launches its kernels one by one, and a mixed step with a long row: the same bits
+    and launches as layers that run one by one, through each decode-attention kernel."""
+    from socrates_b200.engine.model import Model
+    from socrates_b200.engine.runner import StepEntry
+    from socrates_b200.kernels.layer_calls import Recording
+    if how == "64":
+        monkeypatch.setenv("PAGED_PARTITION", "64")
+    if how == "shares":
+        monkeypatch.setattr(Model, "prefers_shares", lambda *a: True)
+    names, runs, run = set(), [], Recording.run
+
+    def seen(self, addresses):
+        runs.append(1)
+        names.update(name for name, _ in self._recorder.calls)
+        return run(self, addresses)
+    monkeypatch.setattr(Recording, "run", seen)
+
+    def last_step():
+        engine = build(torch.bfloat16)
+        g = torch.Generator().manual_seed(6)
+        ids = lambda n: torch.randint(0, 300, (n,), generator=g).tolist()
+        for row, lengths in enumerate([(600, 600), (9,), (300,), (44,)]):
+            engine.cache.assign(row)
+            for i, n in enumerate(lengths):
+                assert engine.cache.reserve(row, sum(lengths[:i + 1]) + 150)
+                engine.runner.step([StepEntry(row, ids(n), sum(lengths[:i]), [n - 1])])
+                engine.cache.commit(row, sum(lengths[:i + 1]))
+        at, before = (1200, 9, 300, 44), len(runs)
+        counts = (1, 1, 130, 1) if how == "mixed" else (1, 1, 1, 1)
+        names.clear()
+        logits = engine.runner.step([StepEntry(r, ids(n), at[r], [n - 1]) for r, n in enumerate(counts)]).logits.clone()
+        return logits, engine.runner.kernel_launches, len(runs) - before
+    got, launches, replayed = last_step()
+    assert replayed == 3 and kernel in names
+    monkeypatch.setattr(Model, "_like_another", lambda *a: False)
+    want, plain, replayed = last_step()
+    assert replayed == 0 and launches == plain and torch.equal(got, want)
 
 
 @pytest.mark.parametrize("change", [
