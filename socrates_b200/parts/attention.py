@@ -221,6 +221,8 @@ class GQAAttention(Part):
         N = len(lengths)
         if N < 5 or paged_partition() is not None:          # few rows are cut into many partitions each: even anyway
             return False
+        if not ops.attention_balanced_supports(self.Hq, self.Hkv, self.D, 16, N):       # (on pages of the usual size)
+            return False
         parts = partitions_in(num_sms * ops.attention_decode_mma_blocks_per_sm(self.D), self.Hkv * N)
         shares = ops.attention_balanced_shares(self.Hq, self.Hkv, self.D, N, num_sms)
         if self.window:

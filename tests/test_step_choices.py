@@ -190,3 +190,13 @@ def test_shares_are_weighed_against_the_partitions_that_the_launch_has(Hkv, leng
     NP = decode_partitions(ctx, Hkv, ops.attention_decode_mma_blocks_per_sm(128), 128)
     longest, total = -(-max(lengths) // 64), sum(lengths) / 64 + N / 2
     assert (-(-longest // NP) - total / ops.attention_balanced_shares(32, Hkv, 128, N, 148) >= 8) == shares
+
+
+@pytest.mark.parametrize("head_dim,N,shares", [(128, 19, True), (256, 19, False), (128, 1024, True), (128, 1025, False)])
+def test_no_shares_where_their_kernel_does_not_serve(head_dim, N, shares):
+    """A step that asked for them would only be recorded a second time, with the same kernels."""
+    from socrates_b200.config.plan import PartSpec
+    from socrates_b200.parts.attention import GQAAttention
+    part = GQAAttention(PartSpec("gqa_attention", dict(hidden_size=64, num_heads=32, num_kv_heads=8, head_dim=head_dim,
+                                                       position=PartSpec("none", {}))), "")
+    assert part.prefers_shares([7001] + [437] * (N - 1), 148) == shares
