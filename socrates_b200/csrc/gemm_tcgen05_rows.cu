@@ -766,7 +766,10 @@ constexpr int persistent_stages(int bn) {
 // of waves times the time of one tile: choose the width for which that is least.  A tile's time
 // per K block was measured at 2,048 x 2,560 x 9,728 (clocks: 659 at width 128, 697 at 160, 780 at
 // 256): narrow tiles save far less than their width, because the 128 rows of A are fetched for
-// each of them and shared memory, not the tensor core, sets the pace.
+// each of them and shared memory, not the tensor core, sets the pace.  These are from when one lane
+// issued the products; with whole warps it is 598, 626 and 736 there, in the same proportions
+// within 5 %, and from 260 to 4,096 rows of the o and down projections of 4B, 8B and 32B the width
+// chosen is within 3 % of the fastest of the three.
 static int pick_bn(int M, int N, int num_sms) {
     const int tiles_m = (M + BM - 1) / BM;
     int best = 256;
@@ -782,7 +785,9 @@ static int pick_bn(int M, int N, int num_sms) {
 
 // Two issuing threads: at width 128 always (four accumulators fit, the epilogue still overlaps
 // the next tile), at 160 only without the SiLU*mul epilogue (one tile at a time there: with the
-// heavier epilogue exposed, gate/up lost 4 %; o and down gain 1 to 10 %).
+// heavier epilogue exposed, gate/up lost 4 %).  Taken again with issuing warps that walk their loops
+// whole, us with two / with one: 2,048 x 2,560 x 9,728 at width 160 96.9 / 98.1, at 128 139 / 143;
+// 512 rows 50.4 / 59.0 and 53.5 / 60.5; 1,999 x 5,120 x 25,600 604 / 612 and 724 / 762.
 constexpr int row_issuers(int bn, int epi) { return bn == 128 || (bn == 160 && epi == 0) ? 2 : 1; }
 
 template <typename TC>

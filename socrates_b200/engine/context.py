@@ -217,7 +217,13 @@ class StepContext:
         panel side by side, so the panel comes from memory once, while equal shares shift every
         pair to another K offset and rely on the cache to keep what an earlier pair fetched
         (measured at 2,048 rows: 2,560 x 9,728, 90 MB of operands, 94 against 116 us; 5,120 x
-        25,600, 367 MB, 525 against 469 us).  Shapes alone decide."""
+        25,600, 367 MB, 525 against 469 us).  Shapes alone decide.
+
+        The costs are from when one lane issued the products.  Since whole warps do, both kinds are faster and whole tiles
+        the more so: into float32, equal shares / the best whole tiles (us), 2,560 x 9,728: 768 rows 43.6 / 39.4, 1,023 50.9 /
+        45.0, 1,500 71.3 / 63.2, 2,048 89.1 / 98.6; 2,560 x 4,096: 1,023 32.3 / 21.0, 2,048 45.4 / 44.9; 4,096 x 4,096: 512
+        26.5 / 19.8, 1,280 42.1 / 44.9.  The rule has equal shares at all of these: a prompt of 1,023 tokens through 18
+        layers of 4B takes 5,754 us with it and 5,243 without (SOCRATES_GEMM_SHARES=0), one of 2,048 9,870 and 9,921."""
         if not self.uses_tensor_cores(x_dtype, w) or os.environ.get("SOCRATES_GEMM_SHARES", "1") == "0":
             return 0
         N, K = w.shape
