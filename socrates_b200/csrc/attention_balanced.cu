@@ -21,7 +21,7 @@
 // requests runs this kernel for the latter and a tile kernel for the former.
 //
 // Measured (us a launch, cold keys, 32 query and 8 KV heads of 128, split-key kernel / this one): 19 rows of 437 to
-// 7,001 keys (257 MB) 110 / 48, i.e. 5.3 TB/s; 64 rows of 256 to 4,096 (572 MB) 124 / 95, 6.0 TB/s.
+// 7,001 keys (257 MB) 110 / 48, i.e. 5.3 TB/s; 64 rows evenly from 256 to 4,096 (572 MB) 109 / 98, 5.9 TB/s.
 #include <math.h>
 
 #include "attention_mma.cuh"
