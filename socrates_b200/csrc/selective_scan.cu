@@ -8,11 +8,13 @@
 // Step sizes, decays, exponentials and the state are float32; x, z, B and C come in the model dtype.
 //
 // A block serves some channels of one request and walks its tokens of the step in order; TS
-// threads share a channel (thread l owns states l, l + TS, ...) and add their parts of y by
-// shuffles in a fixed order.  B and C of a few tokens at a time go through shared memory.
+// threads share a channel and add their parts of y by shuffles in a fixed order.  B and C of a few
+// tokens at a time go through shared memory.  selective_scan_quads_kernel serves the usual numbers of
+// states (8, 16, 32 or 64, four neighbours a thread); selective_scan_kernel every other one.
 #include <math.h>
 
 #include "common.cuh"
+#include "f32x2.cuh"
 
 using namespace sb;
 
@@ -178,6 +180,199 @@ __global__ void __launch_bounds__(THREADS) selective_scan_kernel(ScanArgs a) {
     }
 }
 
+// ----------------------------------------------------------------------------------------
+// The usual numbers of states: TS = 2, 4, 8 or 16 threads a channel with four neighbouring states each, so that a token costs
+// a thread one 16-byte load of B and one of C, two-wide multiply-adds and nothing that is not its own.  What bounds it is the
+// exponential unit (one per state and token, 16 a clock and SM); everything else has to fit beside that:
+//   * the tokens' own values (step size, its product with x, D x, the gate) are made by threads that lie along the channels
+//     (whole lines of dt_raw, x and z), the next sixteen tokens' loads in flight while these are walked;
+//   * A is held times log2(e), so that a decay is one product and one ex2 (bfloat16 engine);
+//   * y is summed for TS tokens at once: each shuffle halves the tokens a lane keeps, so the group's lane l ends with the sum of
+//     token l, gates and stores it (TS - 1 shuffles for TS tokens, the sums in the order of a butterfly).
+// 1,500 tokens by 4,096 channels of 16 states, both passes and the join (bfloat16): 456 us with a thread's states TS apart, a
+// shuffle tree a token and eight predicated states a thread whatever their number, 108 here (the exponentials alone, twice
+// 98 M of them, are 44); 2,048 tokens 652 / 138, 187 tokens of two requests in one launch 99 / 27.
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    sb::fma2(c, a, b);
+    return c;
+}
+__device__ __forceinline__ void unpair(unsigned long long v, float& lo, float& hi) { lo = low(v); hi = high(v); }
+// exp(dt * A) from dt * `unit`: the float32 engine's `unit` is A, the bfloat16 engine's A * log2(e) (see decay_exp)
+template <typename T> __device__ __forceinline__ float decay_unit(float A) { return A; }
+template <> __device__ __forceinline__ float decay_unit<__nv_bfloat16>(float A) { return A * 1.4426950408889634f; }
+template <typename T> __device__ __forceinline__ float decay_of(float x) { return expf(x); }
+template <> __device__ __forceinline__ float decay_of<__nv_bfloat16>(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+template <typename T, int MODE, int TS>
+__global__ void __launch_bounds__(THREADS) selective_scan_quads_kernel(ScanArgs a) {
+    sb::pdl_launch_dependents();
+    constexpr int STATES = 4 * TS;
+    constexpr int CH = THREADS / TS;                        // channels of a block
+    constexpr int ITEMS = TOKENS / TS;                      // (token, channel) values that a thread makes of a stage
+    __shared__ float2 steps[2][TOKENS][CH];                 // dt, dt * x
+    __shared__ float2 gates[MODE == 1 ? 1 : 2][MODE == 1 ? 1 : TOKENS][CH];     // D * x, silu(z)
+    __shared__ __align__(16) float bcs[2][TOKENS * 2 * STATES];
+    const int tid = threadIdx.x;
+    const int l = tid % TS, ch = tid / TS;                  // in the walk: states 4 l .. 4 l + 3 of channel ch
+    const int mc = tid % CH, mt = tid / CH;                 // in the making: channel mc of tokens mt, mt + TS, ...
+    const int c = blockIdx.x * CH + ch;
+    const bool live = c < a.inner;
+    const int cm = blockIdx.x * CH + mc;
+    const bool making = cm < a.inner;
+    float unit[4];
+    {
+        const float4 v = live ? *reinterpret_cast<const float4*>(a.A_log + (size_t)c * STATES + 4 * l) : make_float4(0.f, 0.f, 0.f, 0.f);
+        unit[0] = decay_unit<T>(-expf(v.x));
+        unit[1] = decay_unit<T>(-expf(v.y));
+        unit[2] = decay_unit<T>(-expf(v.z));
+        unit[3] = decay_unit<T>(-expf(v.w));
+    }
+    const unsigned long long unit01 = pair(unit[0], unit[1]), unit23 = pair(unit[2], unit[3]);
+    const float bias = making ? a.dt_bias[cm] : 0.f;
+    const float Dc = making ? a.D[cm] : 0.f;
+    sb::pdl_wait();
+    int r = blockIdx.y, si = 0;
+    if (MODE != 0 && !find_segment(blockIdx.y, a.seq_starts, a.R, a.seg, r, si)) return;
+    const int n0 = MODE == 0 ? a.seq_starts[r] : a.seq_starts[r] + si * a.seg;
+    const int n1 = MODE == 0 ? a.seq_starts[r + 1] : min(a.seq_starts[r + 1], n0 + a.seg);
+    float* st = (MODE == 0 ? a.state + ((size_t)a.seq_rows[r] * a.inner + (live ? c : 0)) * STATES
+                           : a.seg_state + ((size_t)blockIdx.y * a.inner + (live ? c : 0)) * STATES) + 4 * l;
+    unsigned long long S01 = 0ull, S23 = 0ull;
+    if (MODE != 1 && live) {
+        const float4 v = *reinterpret_cast<const float4*>(st);
+        S01 = pair(v.x, v.y);
+        S23 = pair(v.z, v.w);
+    }
+    const T* xs = (const T*)a.x;
+    const T* zs = (const T*)a.z;
+    const T* bc = (const T*)a.bc;
+    float raws[ITEMS];
+    T xv[ITEMS], zv[ITEMS], bv[TS];
+    auto fetch = [&](int t0) {
+        const int nt = min(TOKENS, n1 - t0);
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const int t = mt + k * TS;
+            raws[k] = 0.f;
+            xv[k] = zv[k] = from_float<T>(0.f);
+            if (making && t < nt) {
+                const size_t n = t0 + t;
+                raws[k] = a.dt_raw[n * a.inner + cm];
+                xv[k] = xs[n * a.x_stride + cm];
+                if (MODE != 1) zv[k] = zs[n * a.z_stride + cm];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < TS; ++k) {
+            const int i = tid + k * THREADS, t = i / (2 * STATES), col = i % (2 * STATES);
+            bv[k] = t < nt ? bc[(size_t)(t0 + t) * a.bc_stride + col] : from_float<T>(0.f);
+        }
+    };
+    float dt_sum = 0.f;
+    if (n0 < n1) fetch(n0);
+    int buf = 0;
+    for (int t0 = n0; t0 < n1; t0 += TOKENS, buf ^= 1) {
+        const int nt = min(TOKENS, n1 - t0);
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const int t = mt + k * TS;
+            if (t < nt) {
+                const float raw = raws[k] + bias, x = to_float(xv[k]), z = to_float(zv[k]);
+                const float dt = raw > 20.f ? raw : log1pf(expf(raw));
+                dt_sum += dt;
+                steps[buf][t][mc] = make_float2(dt, dt * x);
+                if constexpr (MODE != 1) gates[buf][t][mc] = make_float2(Dc * x, z / (1.0f + expf(-z)));
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < TS; ++k) bcs[buf][tid + k * THREADS] = to_float(bv[k]);
+        // (one barrier a stage: the buffer that the next stage writes was last read before this one)
+        __syncthreads();
+        if (t0 + TOKENS < n1) fetch(t0 + TOKENS);
+        auto walk = [&](int t) {                            // token t of the stage; the thread's part of its y
+            const float2 v = steps[buf][t][ch];
+            const ulonglong2 B = *reinterpret_cast<const ulonglong2*>(&bcs[buf][t * 2 * STATES + 4 * l]);
+            const unsigned long long dt2 = pair(v.x, v.x), dx2 = pair(v.y, v.y);
+            float e0, e1, e2, e3;
+            unpair(mul2(dt2, unit01), e0, e1);
+            unpair(mul2(dt2, unit23), e2, e3);
+            S01 = fma2(pair(decay_of<T>(e0), decay_of<T>(e1)), S01, mul2(dx2, B.x));
+            S23 = fma2(pair(decay_of<T>(e2), decay_of<T>(e3)), S23, mul2(dx2, B.y));
+            float lo = 0.f, hi = 0.f;
+            if constexpr (MODE != 1) {
+                const ulonglong2 C = *reinterpret_cast<const ulonglong2*>(&bcs[buf][t * 2 * STATES + STATES + 4 * l]);
+                unpair(fma2(S23, C.y, mul2(S01, C.x)), lo, hi);
+            }
+            return lo + hi;
+        };
+#pragma unroll 1
+        for (int tb = 0; tb < nt; tb += TS) {
+            float y[TS];
+            if (tb + TS <= nt) {
+#pragma unroll
+                for (int j = 0; j < TS; ++j) y[j] = walk(tb + j);
+            } else {
+#pragma unroll
+                for (int j = 0; j < TS; ++j) y[j] = tb + j < nt ? walk(tb + j) : 0.f;
+            }
+            if constexpr (MODE != 1) {
+#pragma unroll
+                for (int o = TS >> 1; o > 0; o >>= 1) {
+                    const bool upper = (l & o) != 0;
+#pragma unroll
+                    for (int i = 0; i < o; ++i) {
+                        const float keep = upper ? y[i + o] : y[i], send = upper ? y[i] : y[i + o];
+                        y[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                    }
+                }
+                if (live && tb + l < nt) {
+                    const float2 g = gates[buf][tb + l][ch];
+                    ((T*)a.out)[(size_t)(t0 + tb + l) * a.inner + c] = from_float<T>((y[0] + g.x) * g.y);
+                }
+            }
+        }
+    }
+    if (MODE == 1) {
+        __syncthreads();                                    // everybody is done with the steps
+        float* sums = reinterpret_cast<float*>(steps);      // [TS][CH]
+        sums[mt * CH + mc] = dt_sum;
+        __syncthreads();
+        if (mt == 0 && making) {
+            float s = 0.f;
+#pragma unroll
+            for (int k = 0; k < TS; ++k) s += sums[k * CH + mc];
+            a.seg_dt[(size_t)blockIdx.y * a.inner + cm] = s;
+        }
+    }
+    if (MODE != 2 && live) {
+        float4 v;
+        unpair(S01, v.x, v.y);
+        unpair(S23, v.z, v.w);
+        *reinterpret_cast<float4*>(st) = v;
+    }
+}
+
+template <int MODE> void launch_scan(const ScanArgs& a, dim3 grid, size_t smem, bool quads, int dtype, cudaStream_t stream) {
+    const dim3 block(THREADS);
+#define SB_SCAN(T)                                                                                              \
+    if (!quads) sb::launch(selective_scan_kernel<T, MODE>, grid, block, smem, stream, a);                        \
+    else if (a.TS == 2) sb::launch(selective_scan_quads_kernel<T, MODE, 2>, grid, block, 0, stream, a);          \
+    else if (a.TS == 4) sb::launch(selective_scan_quads_kernel<T, MODE, 4>, grid, block, 0, stream, a);          \
+    else if (a.TS == 8) sb::launch(selective_scan_quads_kernel<T, MODE, 8>, grid, block, 0, stream, a);          \
+    else sb::launch(selective_scan_quads_kernel<T, MODE, 16>, grid, block, 0, stream, a);
+    if (dtype == SB_F32) { SB_SCAN(float) } else { SB_SCAN(__nv_bfloat16) }
+#undef SB_SCAN
+}
+
 // Between MODE 1 and MODE 2: one thread per (channel, state) of a request walks its segments.
 __global__ void __launch_bounds__(256) selective_scan_join_kernel(ScanArgs a) {
     sb::pdl_launch_dependents();
@@ -226,6 +421,10 @@ extern "C" int sb_selective_scan(const void* x, long long x_stride, const void* 
     int TS = 1;
     while (TS * NPT < states) TS *= 2;
     while (TS < 4 && TS * 2 <= states) TS *= 2;
+    // the kernel of neighbouring states: 16-byte pieces of A_log and of the states
+    const bool quads = (states == 8 || states == 16 || states == 32 || states == 64) &&
+                       ((reinterpret_cast<uintptr_t>(A_log) | reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(scratch)) & 15) == 0;
+    if (quads) TS = states / 4;
     ScanArgs a;
     a.x = x; a.x_stride = x_stride; a.z = z; a.z_stride = z_stride; a.dt_raw = dt_raw; a.dt_bias = dt_bias;
     a.bc = bc; a.bc_stride = bc_stride; a.A_log = A_log; a.D = D; a.state = state; a.out = out;
@@ -240,20 +439,13 @@ extern "C" int sb_selective_scan(const void* x, long long x_stride, const void* 
                         (long long)segs * inner * (states + 1) <= scratch_floats;
     a.R = R; a.seg = SEGMENT; a.seg_state = scratch; a.seg_dt = scratch ? scratch + (size_t)segs * inner * states : nullptr;
     if (!spread) {
-        if (dtype == SB_F32) sb::launch(selective_scan_kernel<float, 0>, grid, dim3(THREADS), smem, stream, a);
-        else sb::launch(selective_scan_kernel<__nv_bfloat16, 0>, grid, dim3(THREADS), smem, stream, a);
+        launch_scan<0>(a, grid, smem, quads, dtype, stream);
         SB_LAUNCH_CHECK();
     }
     dim3 sgrid(grid.x, segs), jgrid((inner * states + 255) / 256, R);
-    if (dtype == SB_F32) {
-        sb::launch(selective_scan_kernel<float, 1>, sgrid, dim3(THREADS), smem, stream, a);
-        sb::launch(selective_scan_join_kernel, jgrid, dim3(256), 0, stream, a);
-        sb::launch(selective_scan_kernel<float, 2>, sgrid, dim3(THREADS), smem, stream, a);
-    } else {
-        sb::launch(selective_scan_kernel<__nv_bfloat16, 1>, sgrid, dim3(THREADS), smem, stream, a);
-        sb::launch(selective_scan_join_kernel, jgrid, dim3(256), 0, stream, a);
-        sb::launch(selective_scan_kernel<__nv_bfloat16, 2>, sgrid, dim3(THREADS), smem, stream, a);
-    }
+    launch_scan<1>(a, sgrid, smem, quads, dtype, stream);
+    sb::launch(selective_scan_join_kernel, jgrid, dim3(256), 0, stream, a);
+    launch_scan<2>(a, sgrid, smem, quads, dtype, stream);
     SB_LAUNCH_CHECK();
 }
 
