@@ -13,6 +13,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "f32x2.cuh"
 
 using namespace sb;
 
@@ -412,6 +413,12 @@ __global__ void __launch_bounds__(256) retention_state_scan_kernel(RetChunkArgs 
     }
 }
 
+void launch_state_scan(const RetChunkArgs& ca, cudaStream_t stream) {
+    int slices = (ca.r.dk * ca.r.dv + 255) / 256;
+    if (slices > 64) slices = 64;
+    sb::launch(retention_state_scan_kernel, dim3(ca.r.H, ca.R, slices), dim3(256), 0, stream, ca);
+}
+
 template <typename T, int JJ, int MODE>
 void launch_chunk_mode(const RetChunkArgs& ca, dim3 grid, size_t smem, cudaStream_t stream) {
     static sb::OncePerDevice once;
@@ -430,9 +437,7 @@ void launch_retention_chunked_jj(const RetChunkArgs& ca, int chunks, size_t smem
         return;
     }
     launch_chunk_mode<T, JJ, 1>(ca, dim3(ca.r.H, chunks), smem, stream);
-    int slices = (ca.r.dk * ca.r.dv + 255) / 256;
-    if (slices > 16) slices = 16;
-    sb::launch(retention_state_scan_kernel, dim3(ca.r.H, ca.R, slices), dim3(256), 0, stream, ca);
+    launch_state_scan(ca, stream);
     launch_chunk_mode<T, JJ, 2>(ca, dim3(ca.r.H, chunks), smem, stream);
 }
 
@@ -448,6 +453,349 @@ int launch_retention_chunked(const RetArgs& a, int R, int C, int chunks, float* 
     else if (a.dv <= 256) launch_retention_chunked_jj<T, 8>(ca, chunks, smem, stream);
     else return 1;
     return 0;
+}
+
+// ----------------------------------------------------------------------------------------
+// The three-launch form in register tiles, for the usual heads: dk a multiple of 16 up to 128, dv of 64, 128 or 256, all dims
+// rotating or none, 16-byte pieces.  Same formulas and chunks of 64 tokens, everything float32 on the CUDA cores; what bounds
+// the kernels above is a shared-memory load per four multiply-adds.  Here a thread holds 8 x 8 outputs (tokens or state rows by
+// value columns; two-wide multiply-adds over pairs of tokens), so that four 16-byte loads feed 32 of them, and the operand
+// whose rows are contracted lies transposed (Qt, Kt, At: [contraction][token]).  V takes the state's place in shared memory once
+// Q S0 is done, which leaves room for three blocks an SM at 64 x 128.  Scores above the diagonal are zeros; the products of
+// the chunk's first 32 tokens with its last 32 values are left out.
+// The three launches (bfloat16, 16 heads): 1,500 tokens, 64 x 128: 151 us with the kernels above, 70 with these; 2,048 tokens
+// 180 / 89, 128 x 256 798 / 281, 32 x 64 90 / 48; 200 tokens of 64 x 128 83 / 55.
+constexpr int TC = 64;                  // tokens of a chunk
+constexpr int TPAD = TC + 4;            // floats between the rows of Qt, Kt and At
+
+// 8 consecutive elements, 16-byte aligned
+template <typename T> __device__ __forceinline__ void load8(const T* p, float (&v)[8]) {
+#pragma unroll
+    for (int k = 0; k < 8 / Vec16<T>::N; ++k) {
+        Vec16<T> x;
+        x.load(p + k * Vec16<T>::N);
+#pragma unroll
+        for (int e = 0; e < Vec16<T>::N; ++e) v[k * Vec16<T>::N + e] = x.get(e);
+    }
+}
+// 4 consecutive elements, aligned to their size
+__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
+    const float4 x = *reinterpret_cast<const float4*>(p);
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+}
+__device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&v)[4]) {
+    const uint2 x = *reinterpret_cast<const uint2*>(p);
+    v[0] = __uint_as_float(x.x << 16); v[1] = __uint_as_float(x.x & 0xffff0000u);
+    v[2] = __uint_as_float(x.y << 16); v[3] = __uint_as_float(x.y & 0xffff0000u);
+}
+__device__ __forceinline__ void store4(float* p, const float (&v)[4]) {
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&v)[4]) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+
+// One rotated piece of q or k: dims i0 .. i0 + 7 and their partners half a head on.
+template <typename T>
+__device__ __forceinline__ void load_rotated(const T* row, int i0, int half, bool there, bool turns, const float (&c)[8],
+                                             const float (&s)[8], float scale, float (&lo)[8], float (&hi)[8]) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) lo[e] = hi[e] = 0.f;
+    if (!there) return;
+    load8(row + i0, lo);
+    load8(row + i0 + half, hi);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const float u = lo[e], v = hi[e];
+        if (turns) {
+            lo[e] = u * c[e] - v * s[e];
+            hi[e] = v * c[e] + u * s[e];
+        }
+        lo[e] *= scale;
+        hi[e] *= scale;
+    }
+}
+
+// MODE 1 and 2 as above; a block of 128 threads for each 128 value columns (COLS), NC groups of 4 columns a thread.
+template <typename T, int MODE, int NC, int COLS>
+__global__ void __launch_bounds__(128 * COLS, COLS == 1 ? 3 : 1) retention_tiles_kernel(RetChunkArgs ca) {
+    sb::pdl_launch_dependents();
+    const RetArgs& a = ca.r;
+    constexpr int THR = 128 * COLS, DV = 64 * NC * COLS;
+    extern __shared__ __align__(16) float sm[];
+    const int dk = a.dk, half = dk / 2, rows = (dk + TC - 1) / TC * TC;
+    const int k_stride = MODE == 1 ? rows + 4 : TPAD;
+    float* Ks = sm;                         // MODE 1: [TC][rows + 4] (a token's k along a row); MODE 2: Kt [dk][TPAD], later At [TC][TPAD]
+    float* Qt = Ks + (MODE == 1 ? TC * k_stride : max(dk, TC) * TPAD);       // MODE 2: [dk][TPAD]
+    float* SV = Qt + (MODE == 1 ? 0 : dk * TPAD);                            // [dk][DV] the state, then [TC][DV] the values
+    __shared__ float pw[TC + 1];            // powers of the decay
+    __shared__ float sums[COLS][TC];        // squares of the rows' column halves
+    const int h = blockIdx.x;
+    const int tid = threadIdx.x, tx = tid & 15, ty = (tid >> 4) & 7, part = tid >> 7;
+    const float decay = a.decay[h];
+    if (tid == 0) {
+        float p = 1.f;
+        for (int n = 0; n <= TC; ++n) { pw[n] = p; p *= decay; }
+    }
+    sb::pdl_wait();
+    int r = 0, ci = 0;
+    if (!find_chunk(blockIdx.y, a.seq_starts, ca.R, TC, r, ci)) return;
+    const int c0 = a.seq_starts[r] + ci * TC;
+    const int len = min(TC, a.seq_starts[r + 1] - c0);
+    const int first = a.seq_first_pos[r] + ci * TC;
+    float* S = ca.scratch + ((size_t)blockIdx.y * a.H + h) * dk * DV;
+    const T* in = (const T*)a.qkvg + (size_t)c0 * a.stride;
+    if (MODE == 2)
+        for (int i = tid; i < dk * (DV / 4); i += THR)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(SV + 4 * i))),
+                         "l"(S + 4 * i) : "memory");
+    if (MODE == 1) __syncthreads();         // the powers are there
+    // ---- q and k, rotated; k scaled (and faded to the chunk's end where it makes the state)
+    const bool turns = a.rot != 0;
+    for (int task = tid; task < TC * (dk / 16); task += THR) {
+        const int t = task % TC, i0 = task / TC * 8;
+        float c[8], s[8], lo[8], hi[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (turns) angle_cos_sin((float)(first + t), a.inv_freq[i0 + e], a.inv_freq_lo, i0 + e, c[e], s[e]);
+        const T* row = in + (size_t)t * a.stride;
+        const float scale = MODE == 1 && t < len ? a.k_scale * pw[len - 1 - t] : a.k_scale;
+        load_rotated(row + a.k_off + h * dk, i0, half, t < len, turns, c, s, scale, lo, hi);
+        if (MODE == 1) {
+            float* dst = Ks + t * k_stride + i0;
+            *reinterpret_cast<float4*>(dst) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+            *reinterpret_cast<float4*>(dst + 4) = make_float4(lo[4], lo[5], lo[6], lo[7]);
+            *reinterpret_cast<float4*>(dst + half) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<float4*>(dst + half + 4) = make_float4(hi[4], hi[5], hi[6], hi[7]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                Ks[(i0 + e) * TPAD + t] = lo[e];
+                Ks[(i0 + half + e) * TPAD + t] = hi[e];
+            }
+            load_rotated(row + a.q_off + h * dk, i0, half, t < len, turns, c, s, 1.f, lo, hi);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                Qt[(i0 + e) * TPAD + t] = lo[e];
+                Qt[(i0 + half + e) * TPAD + t] = hi[e];
+            }
+        }
+    }
+    if (MODE == 1)                          // state rows past dk in the last tile
+        for (int i = tid; i < TC * (rows - dk); i += THR) Ks[i / (rows - dk) * k_stride + dk + i % (rows - dk)] = 0.f;
+    // the values of the chunk, zeros past its end
+    constexpr int VECS = TC * DV / 8 / THR;
+    const T* vsrc = in + a.v_off + h * DV;
+    auto put_values = [&](int k, const float (&v)[8]) {
+        float* dst = SV + (tid + k * THR) * 8;
+        *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4*>(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    };
+    auto get_values = [&](int k, float (&v)[8]) {
+        const int i = (tid + k * THR) * 8, t = i / DV;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = 0.f;
+        if (t < len) load8(vsrc + (size_t)t * a.stride + i % DV, v);
+    };
+    unsigned long long acc[4][4 * NC];
+    auto clear = [&]() {
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+#pragma unroll
+            for (int j = 0; j < 4 * NC; ++j) acc[p][j] = 0ull;
+    };
+    const int col = part * 64 * NC + 4 * tx;                 // this thread's columns: col + 64 h + j
+    if constexpr (MODE == 1) {
+#pragma unroll
+        for (int k = 0; k < VECS; ++k) {
+            float v[8];
+            get_values(k, v);
+            put_values(k, v);
+        }
+        __syncthreads();
+        for (int i0 = 0; i0 < rows; i0 += TC) {
+            clear();
+#pragma unroll 4
+            for (int s = 0; s < TC; ++s) tile_step<NC, 0>(acc, Ks + s * k_stride + i0 + 4 * ty, SV + s * DV + col);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                const int i = i0 + 32 * (p >> 1) + 4 * ty + 2 * (p & 1);
+                if (i >= dk) continue;
+#pragma unroll
+                for (int hh = 0; hh < NC; ++hh) {
+                    const unsigned long long* q = &acc[p][4 * hh];
+                    *reinterpret_cast<float4*>(S + (size_t)i * DV + col + 64 * hh) = make_float4(low(q[0]), low(q[1]), low(q[2]), low(q[3]));
+                    *reinterpret_cast<float4*>(S + (size_t)(i + 1) * DV + col + 64 * hh) = make_float4(high(q[0]), high(q[1]), high(q[2]), high(q[3]));
+                }
+            }
+        }
+    } else {
+        __syncthreads();
+        // ---- decayed scores: tokens t = 4 ty + e and 32 + 4 ty + e by keys s = tx + 16 e of this thread's part
+        constexpr int SE = 4 / COLS;
+        {
+            unsigned long long sc[4][SE];
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+#pragma unroll
+                for (int e = 0; e < SE; ++e) sc[p][e] = 0ull;
+            const float* kp = Ks + tx + 16 * SE * part;
+#pragma unroll 4
+            for (int i = 0; i < dk; ++i) {
+                unsigned long long xs[4];
+                *reinterpret_cast<ulonglong2*>(xs) = *reinterpret_cast<const ulonglong2*>(Qt + i * TPAD + 4 * ty);
+                *reinterpret_cast<ulonglong2*>(xs + 2) = *reinterpret_cast<const ulonglong2*>(Qt + i * TPAD + 32 + 4 * ty);
+#pragma unroll
+                for (int e = 0; e < SE; ++e) {
+                    const unsigned long long yy = twice(kp[i * TPAD + 16 * e]);
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) fma2(sc[p][e], xs[p], yy);
+                }
+            }
+            __syncthreads();                // every reader of Kt is done: At takes its place
+#pragma unroll
+            for (int e = 0; e < SE; ++e) {
+                const int s = tx + 16 * (SE * part + e);
+#pragma unroll
+                for (int g = 0; g < 2; ++g) {
+                    float v[4] = {low(sc[2 * g][e]), high(sc[2 * g][e]), low(sc[2 * g + 1][e]), high(sc[2 * g + 1][e])};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int t = 32 * g + 4 * ty + j;
+                        v[j] = s <= t ? v[j] * pw[t - s] : 0.f;
+                    }
+                    *reinterpret_cast<float4*>(Ks + s * TPAD + 32 * g + 4 * ty) = make_float4(v[0], v[1], v[2], v[3]);
+                }
+            }
+        }
+        // ---- what the state before the chunk gives; the values are on their way meanwhile
+        float early[sizeof(T) == 2 ? VECS : 1][8];
+        if constexpr (sizeof(T) == 2) {
+#pragma unroll
+            for (int k = 0; k < VECS; ++k) get_values(k, early[k]);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();                    // the state and At are there
+        clear();
+#pragma unroll 4
+        for (int i = 0; i < dk; ++i) tile_step<NC, 0>(acc, Qt + i * TPAD + 4 * ty, SV + i * DV + col);
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const int t = 32 * (p >> 1) + 4 * ty + 2 * (p & 1);
+            const float f0 = pw[t + 1], f1 = pw[t + 2 <= TC ? t + 2 : TC];
+#pragma unroll
+            for (int j = 0; j < 4 * NC; ++j) {
+                const float x = low(acc[p][j]) * f0, y = high(acc[p][j]) * f1;
+                acc[p][j] = pair(x, y);
+            }
+        }
+        __syncthreads();                    // every reader of the state is done: the values take its place
+#pragma unroll
+        for (int k = 0; k < VECS; ++k) {
+            if constexpr (sizeof(T) == 2) {
+                put_values(k, early[k]);
+            } else {
+                float v[8];
+                get_values(k, v);
+                put_values(k, v);
+            }
+        }
+        __syncthreads();
+        // ---- and the chunk's own tokens
+#pragma unroll 4
+        for (int s = 0; s < TC / 2; ++s) tile_step<NC, 0>(acc, Ks + s * TPAD + 4 * ty, SV + s * DV + col);
+#pragma unroll 4
+        for (int s = TC / 2; s < TC; ++s) tile_step<NC, 2>(acc, Ks + s * TPAD + 4 * ty, SV + s * DV + col);
+        // ---- norm over the head, gate, store
+        float ss[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            float v = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4 * NC; ++j) {
+                const float x = (k & 1) ? high(acc[k >> 1][j]) : low(acc[k >> 1][j]);
+                v = fmaf(x, x, v);
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            ss[k] = v;
+        }
+        if constexpr (COLS > 1) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (tx == 0) sums[part][32 * (k >> 2) + 4 * ty + (k & 3)] = ss[k];
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int t = 32 * (k >> 2) + 4 * ty + (k & 3);
+                ss[k] = 0.f;
+#pragma unroll
+                for (int q = 0; q < COLS; ++q) ss[k] += sums[q][t];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int t = 32 * (k >> 2) + 4 * ty + (k & 3);
+            if (t >= len) continue;
+            const float rinv = 1.0f / sqrtf(ss[k] / (float)DV + a.eps);
+#pragma unroll
+            for (int hh = 0; hh < NC; ++hh) {
+                float g[4], o[4];
+                load4(in + (size_t)t * a.stride + a.g_off + h * DV + col + 64 * hh, g);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float x = (k & 1) ? high(acc[k >> 1][4 * hh + j]) : low(acc[k >> 1][4 * hh + j]);
+                    o[j] = x * rinv * (g[j] / (1.0f + expf(-g[j])));
+                }
+                store4((T*)a.out + ((size_t)(c0 + t) * a.H + h) * DV + col + 64 * hh, o);
+            }
+        }
+    }
+}
+
+size_t tiles_smem(int mode, int dk, int dv) {
+    const int rows = (dk + TC - 1) / TC * TC;
+    const int sv = (mode == 1 ? TC : (dk > TC ? dk : TC)) * dv;
+    return (size_t)(sv + (mode == 1 ? TC * (rows + 4) : (dk > TC ? dk : TC) * TPAD + dk * TPAD)) * sizeof(float);
+}
+
+template <typename T, int MODE, int NC, int COLS>
+void launch_tiles_mode(const RetChunkArgs& ca, int chunks, cudaStream_t stream) {
+    static sb::OncePerDevice once;
+    if (!once.flag()) {
+        cudaFuncSetAttribute(retention_tiles_kernel<T, MODE, NC, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        once.flag() = true;
+    }
+    sb::launch(retention_tiles_kernel<T, MODE, NC, COLS>, dim3(ca.r.H, chunks), dim3(128 * COLS), tiles_smem(MODE, ca.r.dk, ca.r.dv),
+               stream, ca);
+}
+
+template <typename T, int NC, int COLS>
+void launch_tiles(const RetChunkArgs& ca, int chunks, cudaStream_t stream) {
+    launch_tiles_mode<T, 1, NC, COLS>(ca, chunks, stream);
+    launch_state_scan(ca, stream);
+    launch_tiles_mode<T, 2, NC, COLS>(ca, chunks, stream);
+}
+
+// Whether the tile kernels take a step: head sizes, rotation and 16-byte pieces everywhere.
+bool tiles_take(const RetArgs& a, const float* scratch, int elem) {
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(a.qkvg) | reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(scratch);
+    return (a.dv == 64 || a.dv == 128 || a.dv == 256) && a.dk % 16 == 0 && a.dk <= 128 && (a.rot == 0 || a.rot == a.dk) &&
+           (bits & 15) == 0 && (a.stride * elem) % 16 == 0 && a.q_off * elem % 16 == 0 && a.k_off * elem % 16 == 0 &&
+           a.v_off * elem % 16 == 0 && a.g_off * elem % 16 == 0;
+}
+
+template <typename T>
+void launch_retention_tiles(const RetArgs& a, int R, int chunks, float* scratch, cudaStream_t stream) {
+    RetChunkArgs ca;
+    ca.r = a;
+    ca.C = TC;
+    ca.R = R;
+    ca.scratch = scratch;
+    if (a.dv == 64) launch_tiles<T, 1, 1>(ca, chunks, stream);
+    else if (a.dv == 128) launch_tiles<T, 2, 1>(ca, chunks, stream);
+    else launch_tiles<T, 2, 2>(ca, chunks, stream);
 }
 
 }  // namespace
@@ -477,6 +825,12 @@ extern "C" int sb_retention(const void* qkvg, long long stride, int q_off, int k
             const int chunks = (N + C - 1) / C + R;
             const bool spread = scratch != nullptr && R * H < 132 && chunks > 2 * R &&
                                 (long long)chunks * H * dk * dv <= scratch_floats;
+            const int tiles = (N + TC - 1) / TC + R;        // (the tile kernels' chunks, never more than the others')
+            if (spread && tiles_take(a, scratch, dtype == SB_F32 ? 4 : 2)) {
+                if (dtype == SB_F32) launch_retention_tiles<float>(a, R, tiles, scratch, stream);
+                else launch_retention_tiles<__nv_bfloat16>(a, R, tiles, scratch, stream);
+                SB_LAUNCH_CHECK();
+            }
             int bad = 1;
             if (dtype == SB_F32) bad = launch_retention_chunked<float>(a, R, C, chunks, spread ? scratch : nullptr, need(C), stream);
             else if (dtype == SB_BF16)
