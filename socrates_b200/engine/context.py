@@ -210,20 +210,19 @@ class StepContext:
         is partial sums should run on it, else 0.  Whole tiles run in waves over the SMs; a product
         whose last wave is mostly empty (a 2,048-row portion through a 2,560-wide projection: 80
         tiles of 256 x 256 for 74 pairs, 256 tiles of 128 x 160 for 148 SMs) loses up to half of
-        its time there.  Chosen when the model of the kernels' measured costs per K block (690
-        clocks for a pair's 256 x 256 tile; 540 + 0.94 * width for one SM's 128 x width tile) says
-        that equal shares take less than 0.9 of the best whole-tile choice, and both operands
-        together stay well inside the L2 cache (96 MB): whole tiles run the row tiles of a weight
-        panel side by side, so the panel comes from memory once, while equal shares shift every
-        pair to another K offset and rely on the cache to keep what an earlier pair fetched
-        (measured at 2,048 rows: 2,560 x 9,728, 90 MB of operands, 94 against 116 us; 5,120 x
-        25,600, 367 MB, 525 against 469 us).  Shapes alone decide.
+        its time there.  Both operands together stay well inside the L2 cache (96 MB): whole tiles run the
+        row tiles of a weight panel side by side, so the panel comes from memory once, while equal shares
+        shift every pair to another K offset and rely on the cache to keep what an earlier pair fetched
+        (measured at 2,048 rows: 2,560 x 9,728, 90 MB of operands, 89 against 99 us; 5,120 x 25,600, 367 MB,
+        525 against 469 us).  Shapes alone decide.
 
-        The costs are from when one lane issued the products.  Since whole warps do, both kinds are faster and whole tiles
-        the more so: into float32, equal shares / the best whole tiles (us), 2,560 x 9,728: 768 rows 43.6 / 39.4, 1,023 50.9 /
-        45.0, 1,500 71.3 / 63.2, 2,048 89.1 / 98.6; 2,560 x 4,096: 1,023 32.3 / 21.0, 2,048 45.4 / 44.9; 4,096 x 4,096: 512
-        26.5 / 19.8, 1,280 42.1 / 44.9.  The rule has equal shares at all of these: a prompt of 1,023 tokens through 18
-        layers of 4B takes 5,754 us with it and 5,243 without (SOCRATES_GEMM_SHARES=0), one of 2,048 9,870 and 9,921."""
+        Equal shares cost 13.9 us and 0.455 for each K block of a pair's share; whole tiles 7 us and, a K block and wave,
+        0.215 / 0.26 / 0.365 at widths of 128 / 160 / 256 while there is one wave, 0.27 / 0.297 / 0.357 beyond, when the GPU is
+        full (fits within 8 % of what 260 to 4,096 rows through the o and down projections of 4B, 8B and 32B take into
+        float32).  Measured, equal shares / the best whole tiles (us): 2,560 x 9,728: 640 rows 42.3 / 40.1, 1,023 50.9 / 45.0,
+        1,280 58.7 / 62.2, 1,500 71.3 / 63.2, 2,048 89.1 / 98.6; 2,560 x 4,096: 1,023 32.3 / 21.0, 2,048 45.4 / 44.9; 4,096 x 4,096:
+        512 26.5 / 19.8, 1,023 36.9 / 29.7, 1,280 42.1 / 44.9, 1,500 47.6 / 52.2, 1,792 53.3 / 52.6; 5,120 x 8,192: 512 48.1 / 41.9,
+        1,023 74.4 / 85.3."""
         if not self.uses_tensor_cores(x_dtype, w) or os.environ.get("SOCRATES_GEMM_SHARES", "1") == "0":
             return 0
         N, K = w.shape
@@ -233,12 +232,16 @@ class StepContext:
         if parts == 0:
             return 0
         pairs = max(1, self.num_sms // 2)
-        shares_cost = (-(-M // 256) * -(-N // 256)) * 690.0 / pairs
-        rows128 = -(-M // 128)
-        whole_cost = min((-(-(rows128 * -(-N // bn)) // self.num_sms)) * (540.0 + 0.94 * bn) for bn in (256, 160, 128))
+        kb, rows128 = -(-K // 64), -(-M // 128)
+        shares_cost = 13.9 + 0.455 * kb * -(-M // 256) * -(-N // 256) / pairs
+
+        def whole(waves, one, more):
+            return 7.0 + kb * waves * (one if waves == 1 else more)
+        whole_cost = min(whole(-(-(rows128 * -(-N // bn)) // self.num_sms), one, more)
+                         for bn, one, more in ((128, 0.215, 0.27), (160, 0.26, 0.297), (256, 0.365, 0.357)))
         if M >= 4096:       # the pair kernel with whole tiles is the choice there
-            whole_cost = min(whole_cost, (-(-(-(-M // 256) * -(-N // 256)) // pairs)) * 690.0)
-        return parts if shares_cost < 0.9 * whole_cost else 0
+            whole_cost = min(whole_cost, whole(-(-(-(-M // 256) * -(-N // 256)) // pairs), 0.34, 0.34))
+        return parts if shares_cost < 1.02 * whole_cost else 0
 
     def can_fuse_silu_mul(self, M: int, w: torch.Tensor, x_dtype: torch.dtype) -> bool:
         """Whether the product with an interleaved gate/up matrix can apply the gated unit (SiLU or gelu) in its
