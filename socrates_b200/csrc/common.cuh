@@ -157,4 +157,28 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
     return scratch[32];
 }
 
+// Sum over a block of WARPS warps with ONE barrier; `slot` is WARPS floats of shared memory that nothing else uses (a slot
+// per sum).  The order of additions is fixed.
+template <int WARPS> __device__ __forceinline__ float block_sum_once(float v, float* slot) {
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) slot[threadIdx.x >> 5] = v;
+    __syncthreads();
+    float t = slot[0];
+#pragma unroll
+    for (int w = 1; w < WARPS; ++w) t += slot[w];
+    return t;
+}
+
+// 4 floats to 4 elements of T, aligned to their size.
+__device__ __forceinline__ void store_four(float* p, float a, float b, float c, float d) {
+    *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
+}
+__device__ __forceinline__ void store_four(__nv_bfloat16* p, float a, float b, float c, float d) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, d);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+}
+// u += p, by element
+__device__ __forceinline__ void add4(float4& u, const float4& p) { u.x += p.x; u.y += p.y; u.z += p.z; u.w += p.w; }
+__device__ __forceinline__ float squares4(const float4& u) { return u.x * u.x + u.y * u.y + u.z * u.z + u.w * u.w; }
+
 }  // namespace sb

@@ -196,6 +196,83 @@ __global__ void __launch_bounds__(DEPTH > 8 ? 640 : 768) add_rmsnorm_vec_kernel(
     }
 }
 
+// The same for many rows (prompt portions): a row is V float4 columns of each of THR threads, held in registers from the loads to
+// the store, with the residual and the first two partial sums of all of them in flight at once and one barrier a row.  What
+// bounds many rows is memory, once enough loads are under way.
+// With a column or three a thread, the row in shared memory and block_sum's barriers / so (us): 2,048 rows of 2,560 with two
+// parts (94 MB) 25.0 / 15.0, with one 15.6 / 12.3, 5,120 wide with two 43.0 / 29.2; 1,000 rows of 4,096 with one 13.6 / 10.1; 187 of
+// 2,560 with one 3.9 / 2.9, 65 2.5 / 2.5.
+template <typename T, int V, int THR>
+__global__ void __launch_bounds__(THR) add_rmsnorm_rows_kernel(float* __restrict__ residual, const float* __restrict__ delta, int S,
+                                                               size_t delta_stride, const float* __restrict__ gain,
+                                                               T* __restrict__ out, const int* __restrict__ row_index, int d,
+                                                               float eps, int write_residual) {
+    sb::pdl_launch_dependents();
+    __shared__ float slot[THR / 32];
+    const int m = blockIdx.x, d4 = d / 4, tid = threadIdx.x;
+    sb::pdl_wait();
+    const int r = row_index ? row_index[m] : m;
+    float4* res4 = reinterpret_cast<float4*>(residual + (size_t)r * d);
+    const float4* del4 = reinterpret_cast<const float4*>(delta + (size_t)r * d);
+    const size_t stride4 = delta_stride / 4;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v[V], p[V], q[V];
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+        const int i = tid + c * THR;
+        v[c] = p[c] = q[c] = zero;
+        if (i < d4) {
+            v[c] = res4[i];
+            if (S > 0) p[c] = __ldg(del4 + i);
+            if (S > 1) q[c] = __ldg(del4 + stride4 + i);
+        }
+    }
+    if (S > 0) {
+#pragma unroll
+        for (int c = 0; c < V; ++c) add4(v[c], p[c]);
+    }
+    if (S > 1) {
+#pragma unroll
+        for (int c = 0; c < V; ++c) add4(v[c], q[c]);
+    }
+    for (int s = 2; s < S; ++s) {                            // added in the order s = 0, 1, ...
+#pragma unroll
+        for (int c = 0; c < V; ++c)
+            if (tid + c * THR < d4) p[c] = __ldg(del4 + (size_t)s * stride4 + tid + c * THR);
+#pragma unroll
+        for (int c = 0; c < V; ++c) add4(v[c], p[c]);
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+        const int i = tid + c * THR;
+        if (write_residual && i < d4) res4[i] = v[c];
+        if (i < d4) ss += squares4(v[c]);
+    }
+    const float rinv = 1.0f / sqrtf(block_sum_once<THR / 32>(ss, slot) / (float)d + eps);
+    const float4* gain4 = reinterpret_cast<const float4*>(gain);
+    T* o = out + (size_t)m * d;
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+        const int i = tid + c * THR;
+        if (i >= d4) continue;
+        const float4 g = __ldg(gain4 + i);
+        store_four(o + 4 * i, v[c].x * rinv * g.x, v[c].y * rinv * g.y, v[c].z * rinv * g.z, v[c].w * rinv * g.w);
+    }
+}
+
+// V and THR for a row of d4 columns; false: it is too wide for registers.
+template <typename T, typename... Args> bool launch_norm_rows(int M, int d4, cudaStream_t stream, Args... args) {
+#define SB_ROWS(V_, THR_)                                                                                                \
+    if (d4 <= V_ * THR_) {                                                                                               \
+        sb::launch(add_rmsnorm_rows_kernel<T, V_, THR_>, dim3(M), dim3(THR_), 0, stream, args...);                         \
+        return true;                                                                                                     \
+    }
+    SB_ROWS(2, 128) SB_ROWS(4, 128) SB_ROWS(5, 128) SB_ROWS(6, 128) SB_ROWS(4, 256) SB_ROWS(5, 256) SB_ROWS(6, 256) SB_ROWS(8, 256)
+#undef SB_ROWS
+    return false;
+}
+
 // the output pointer type of a norm kernel instantiation (its first template argument)
 template <typename T, int DEPTH = 0> T* sb_out_type();
 
@@ -215,6 +292,11 @@ extern "C" int sb_add_rmsnorm(float* residual, const float* delta, int S, long l
     // regime, where the S partial sums of a column should all be in flight at once; so are 65 to 256
     // rows behind a product in many parts)
     const bool deep = M <= 64 || (M <= 256 && S > 2);
+    // many rows: in registers.  (Float32 rows keep the kernels of few rows, for the order of a row's squares.)
+    if (vec && !deep && dtype == SB_BF16 &&
+        launch_norm_rows<__nv_bfloat16>(M, d / 4, stream, residual, delta, S, (size_t)delta_stride, gain, (__nv_bfloat16*)out,
+                                        row_index, d, eps, write_residual))
+        SB_LAUNCH_CHECK();
     int threads = d >= 2048 ? 512 : 256;
     if (vec) {
         threads = ((d / 4 + 31) / 32) * 32;

@@ -210,6 +210,109 @@ __global__ void __launch_bounds__(512) fold_rmsnorm_vec_kernel(FoldArgs a) {
     }
 }
 
+// A row's columns of a thread: the S partial sums of V float4 columns added in order, DEPTH parts of all V in flight.
+template <int V, int THR, int DEPTH>
+__device__ __forceinline__ void sum_parts(float4 (&b)[V], const float* parts, int S, size_t stride, size_t row, int d4) {
+    const float4* p4 = reinterpret_cast<const float4*>(parts) + row * d4;
+    const size_t stride4 = stride / 4;
+#pragma unroll
+    for (int c = 0; c < V; ++c) b[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s0 = 0; s0 < S; s0 += DEPTH) {
+        float4 p[DEPTH][V];
+#pragma unroll
+        for (int j = 0; j < DEPTH; ++j)
+#pragma unroll
+            for (int c = 0; c < V; ++c) {
+                const int i = threadIdx.x + c * THR;
+                p[j][c] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (i < d4 && s0 + j < S) p[j][c] = __ldg(p4 + (size_t)(s0 + j) * stride4 + i);
+            }
+#pragma unroll
+        for (int j = 0; j < DEPTH; ++j)
+#pragma unroll
+            for (int c = 0; c < V; ++c)
+                if (s0 + j < S) add4(b[c], p[j][c]);
+    }
+}
+template <int V, int THR> __device__ __forceinline__ float squares(const float4 (&b)[V], int d4) {
+    float ss = 0.f;
+#pragma unroll
+    for (int c = 0; c < V; ++c)
+        if (threadIdx.x + c * THR < d4) ss += squares4(b[c]);
+    return ss;
+}
+// v[c] <- f(v[c], the column's float4 of t) for the columns there are
+template <int V, int THR, typename F> __device__ __forceinline__ void with_columns(float4 (&v)[V], const float* t, int d4, F f) {
+    const float4* t4 = reinterpret_cast<const float4*>(t);
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+        const int i = threadIdx.x + c * THR;
+        if (i < d4) f(v[c], __ldg(t4 + i));
+    }
+}
+
+// fold_rmsnorm for many rows: a row is V float4 columns of each of THR threads and stays in registers, with the residual on
+// its way while the branch is normed and one barrier a sum (above, the row goes through shared memory and the residual is
+// loaded after the branch's norm).
+// The kernel above / this one (us), two parts with a gain: 2,048 rows of 2,048 39.7 / 16.2, 1,500 31.9 / 12.9, 300 9.6 / 4.3, 65
+// 4.1 / 3.7.
+template <typename T, int V, int THR>
+__global__ void __launch_bounds__(THR) fold_rmsnorm_rows_kernel(FoldArgs a) {
+    sb::pdl_launch_dependents();
+    __shared__ float slot[2][THR / 32];
+    const int m = blockIdx.x, d4 = a.d / 4, tid = threadIdx.x;
+    sb::pdl_wait();
+    const int r = a.row_index ? a.row_index[m] : m;
+    float4* res4 = reinterpret_cast<float4*>(a.residual + (size_t)r * a.d);
+    const bool branch = a.S > 0 || a.branch_bias != nullptr;
+    float4 v[V], b[V];
+#pragma unroll
+    for (int c = 0; c < V; ++c) v[c] = tid + c * THR < d4 ? res4[tid + c * THR] : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (branch) {
+        sum_parts<V, THR, 2>(b, a.delta, a.S, a.delta_stride, r, d4);
+        if (a.branch_bias) with_columns<V, THR>(b, a.branch_bias, d4, [](float4& u, const float4& t) { add4(u, t); });
+        if (a.branch_gain) {
+            const float binv = 1.0f / sqrtf(block_sum_once<THR / 32>(squares<V, THR>(b, d4), slot[0]) / (float)a.d + a.branch_eps);
+            with_columns<V, THR>(b, a.branch_gain, d4, [&](float4& u, const float4& t) {
+                u.x *= binv * t.x; u.y *= binv * t.y; u.z *= binv * t.z; u.w *= binv * t.w;
+            });
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+        v[c].x *= a.res_scale; v[c].y *= a.res_scale; v[c].z *= a.res_scale; v[c].w *= a.res_scale;
+        if (branch) add4(v[c], b[c]);
+    }
+    if (a.add_rows) with_columns<V, THR>(v, a.add_rows + (size_t)r * a.d, d4, [](float4& u, const float4& t) { add4(u, t); });
+    if (a.add_vec) with_columns<V, THR>(v, a.add_vec, d4, [](float4& u, const float4& t) { add4(u, t); });
+    if (a.write_residual) {
+#pragma unroll
+        for (int c = 0; c < V; ++c)
+            if (tid + c * THR < d4) res4[tid + c * THR] = v[c];
+    }
+    if (a.out == nullptr && !a.norm_residual) return;
+    const bool squash = a.tanh_alpha != nullptr, normed = a.gain != nullptr && !squash;
+    const float alpha = squash ? *a.tanh_alpha : 0.f;
+    const float rinv = normed ? 1.0f / sqrtf(block_sum_once<THR / 32>(squares<V, THR>(v, d4), slot[1]) / (float)a.d + a.eps) : 1.0f;
+    T* o = (T*)a.out + (size_t)m * a.d;
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+        const int i = tid + c * THR;
+        if (i >= d4) continue;
+        float4 x = v[c];
+        if (squash) {
+            const float4 g = __ldg(reinterpret_cast<const float4*>(a.gain) + i), t = __ldg(reinterpret_cast<const float4*>(a.tanh_bias) + i);
+            x = make_float4(fmaf(tanhf(alpha * x.x), g.x, t.x), fmaf(tanhf(alpha * x.y), g.y, t.y),
+                            fmaf(tanhf(alpha * x.z), g.z, t.z), fmaf(tanhf(alpha * x.w), g.w, t.w));
+        } else if (normed) {
+            const float4 g = __ldg(reinterpret_cast<const float4*>(a.gain) + i);
+            x = make_float4(x.x * rinv * g.x, x.y * rinv * g.y, x.z * rinv * g.z, x.w * rinv * g.w);
+        }
+        if (a.norm_residual) res4[i] = x;
+        if (a.out != nullptr) store_four(o + 4 * i, x.x, x.y, x.z, x.w);
+    }
+}
+
 struct MeanArgs {
     const float* x[2];
     int S[2];
@@ -252,6 +355,46 @@ __global__ void __launch_bounds__(256) normed_mean_kernel(MeanArgs a) {
             a.scale * (rows[i] * inv[0] * a.gain[0][i] + rows[d + i] * inv[1] * a.gain[1][i]);
 }
 
+// The same for rows whose columns fit the registers of THR threads (see fold_rmsnorm_rows_kernel); DEPTH parts of a branch in
+// flight, two for many rows.  A row's bits do not depend on it, nor on the number of rows.  The kernel above / this one (us),
+// three parts each: 1,500 rows of 2,048 57.7 / 12.3, 8 rows 9.7 / 3.3.
+template <int V, int THR, int DEPTH>
+__global__ void __launch_bounds__(THR) normed_mean_rows_kernel(MeanArgs a) {
+    sb::pdl_launch_dependents();
+    __shared__ float slot[2][THR / 32];
+    const int d4 = a.d / 4;
+    sb::pdl_wait();
+    float4 x[2][V];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) sum_parts<V, THR, DEPTH>(x[t], a.x[t], a.S[t], a.stride[t], blockIdx.x, d4);
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const float inv = 1.0f / sqrtf(block_sum_once<THR / 32>(squares<V, THR>(x[t], d4), slot[t]) / (float)a.d + a.eps);
+        with_columns<V, THR>(x[t], a.gain[t], d4, [&](float4& u, const float4& g) {
+            u.x = u.x * inv * g.x; u.y = u.y * inv * g.y; u.z = u.z * inv * g.z; u.w = u.w * inv * g.w;
+        });
+    }
+    float* o = a.out + (size_t)blockIdx.x * a.d;
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+        const int i = threadIdx.x + c * THR;
+        if (i < d4)
+            store_four(o + 4 * i, a.scale * (x[0][c].x + x[1][c].x), a.scale * (x[0][c].y + x[1][c].y),
+                       a.scale * (x[0][c].z + x[1][c].z), a.scale * (x[0][c].w + x[1][c].w));
+    }
+}
+
+// Columns a thread and threads for rows of d4 float4 columns: CALL(V, THR); nothing where the rows are too wide.
+#define SB_FOR_ROWS(d4, CALL)                                                                                      \
+    do {                                                                                                           \
+        if ((d4) <= 2 * 128) { CALL(2, 128); }                                                                     \
+        else if ((d4) <= 4 * 128) { CALL(4, 128); }                                                                \
+        else if ((d4) <= 5 * 128) { CALL(5, 128); }                                                                \
+        else if ((d4) <= 4 * 256) { CALL(4, 256); }                                                                \
+        else if ((d4) <= 5 * 256) { CALL(5, 256); }                                                                \
+        else if ((d4) <= 8 * 256) { CALL(8, 256); }                                                                \
+    } while (0)
+
 __device__ __forceinline__ float activation(float z, int act) {
     switch (act) {
         case 1: { const float p = fmaxf(z, 0.f); return p * p; }                       // relu squared
@@ -277,6 +420,45 @@ __global__ void __launch_bounds__(256) bias_act_kernel(T* __restrict__ out, cons
         }
         if (bias) z += bias[i % F];
         out[i] = from_float<T>(activation(z, act));
+    }
+}
+
+// The same with 16-byte accesses (F in whole pieces of 8, aligned rows) for many values, where the accesses count: 2,048 rows
+// of 5,120 24.5 -> 15.3 us, 512 of 2,560 4.3 -> 3.6; 256 of 4,096 3.6 / 3.7, 8 of 2,560 1.5 / 1.9.
+template <typename T>
+__global__ void __launch_bounds__(256) bias_act_vec_kernel(T* __restrict__ out, const T* __restrict__ in,
+                                                           const float* __restrict__ parts, int S, size_t part_stride,
+                                                           const float* __restrict__ bias, int F8, size_t total8, int act) {
+    sb::pdl_launch_dependents();
+    sb::pdl_wait();
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total8; i += (size_t)gridDim.x * blockDim.x) {
+        float z[8];
+        if (parts) {
+            float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+            for (int s = 0; s < S; ++s) {
+                const float4* p = reinterpret_cast<const float4*>(parts + s * part_stride + 8 * i);
+                add4(lo, p[0]);
+                add4(hi, p[1]);
+            }
+            z[0] = lo.x; z[1] = lo.y; z[2] = lo.z; z[3] = lo.w; z[4] = hi.x; z[5] = hi.y; z[6] = hi.z; z[7] = hi.w;
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; k += Vec16<T>::N) {
+                Vec16<T> x;
+                x.load(in + 8 * i + k);
+#pragma unroll
+                for (int e = 0; e < Vec16<T>::N; ++e) z[k + e] = x.get(e);
+            }
+        }
+        if (bias) {
+            const float* b = bias + 8 * (total8 >> 32 ? (int)(i % F8) : (int)((uint32_t)i % (uint32_t)F8));
+#pragma unroll
+            for (int e = 0; e < 8; ++e) z[e] += __ldg(b + e);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) z[e] = activation(z[e], act);
+        store_four(out + 8 * i, z[0], z[1], z[2], z[3]);
+        store_four(out + 8 * i + 4, z[4], z[5], z[6], z[7]);
     }
 }
 
@@ -311,6 +493,14 @@ extern "C" int sb_fold_rmsnorm(float* residual, const float* delta, int S, long 
     const bool vec = d % 4 == 0 && delta_stride % 4 == 0 && aligned(residual) && aligned(delta) && aligned(branch_bias) &&
                      aligned(branch_gain) && aligned(add_rows) && aligned(add_vec) && aligned(gain) && aligned(tanh_bias) &&
                      aligned(out);
+    // many rows of few parts: in registers.  (Few rows want every part of a column in flight; float32 rows keep to the one
+    // kernel in any batch, for the order of their squares.)
+    if (vec && M > 64 && S <= 4 && out_dtype == SB_BF16 && d <= 8192) {
+#define SB_FOLD(V_, THR_) sb::launch(fold_rmsnorm_rows_kernel<__nv_bfloat16, V_, THR_>, dim3(M), dim3(THR_), 0, stream, a)
+        SB_FOR_ROWS(d / 4, SB_FOLD);
+#undef SB_FOLD
+        SB_LAUNCH_CHECK();
+    }
     if (vec) {
         int threads = ((d / 4 + 31) / 32) * 32;
         if (threads > 512) threads = 512;
@@ -353,6 +543,16 @@ extern "C" int sb_normed_mean(float* out, const float* x0, int S0, long long str
     a.x[0] = x0; a.S[0] = S0; a.stride[0] = (size_t)stride0; a.gain[0] = gain0;
     a.x[1] = x1; a.S[1] = S1; a.stride[1] = (size_t)stride1; a.gain[1] = gain1;
     a.out = out; a.d = d; a.eps = eps; a.scale = scale;
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(x0) | reinterpret_cast<uintptr_t>(x1) |
+                           reinterpret_cast<uintptr_t>(gain0) | reinterpret_cast<uintptr_t>(gain1);
+    if (d % 4 == 0 && d <= 8192 && stride0 % 4 == 0 && stride1 % 4 == 0 && (bits & 15) == 0) {
+#define SB_MEAN(V_, THR_)                                                                                            \
+        if (N > 64) sb::launch(normed_mean_rows_kernel<V_, THR_, 2>, dim3(N), dim3(THR_), 0, stream, a);             \
+        else sb::launch(normed_mean_rows_kernel<V_, THR_, (V_ <= 4 ? 8 : V_ == 5 ? 4 : 2)>, dim3(N), dim3(THR_), 0, stream, a)
+        SB_FOR_ROWS(d / 4, SB_MEAN);
+#undef SB_MEAN
+        SB_LAUNCH_CHECK();
+    }
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(normed_mean_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     sb::launch(normed_mean_kernel, dim3(N), dim3(256), smem, stream, a);
@@ -366,6 +566,18 @@ extern "C" int sb_bias_act(void* out, const void* in, const float* parts, int S,
     SB_REQUIRE((in != nullptr) != (parts != nullptr), "bias_act: one input, a matrix or partial sums");
     if (N == 0) return 0;
     const size_t total = (size_t)N * F;
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(parts);
+    if (total >= (5u << 18) && F % 8 == 0 && part_stride % 4 == 0 && (bits & 15) == 0 && (dtype == SB_F32 || dtype == SB_BF16)) {
+        const size_t total8 = total / 8;
+        const int vblocks = (int)((total8 + 255) / 256 < 148 * 8 ? (total8 + 255) / 256 : 148 * 8);
+        if (dtype == SB_F32)
+            sb::launch(bias_act_vec_kernel<float>, dim3(vblocks), dim3(256), 0, stream, (float*)out, (const float*)in, parts, S,
+                       (size_t)part_stride, bias, F / 8, total8, act);
+        else
+            sb::launch(bias_act_vec_kernel<__nv_bfloat16>, dim3(vblocks), dim3(256), 0, stream, (__nv_bfloat16*)out,
+                       (const __nv_bfloat16*)in, parts, S, (size_t)part_stride, bias, F / 8, total8, act);
+        SB_LAUNCH_CHECK();
+    }
     const int blocks = (int)((total + 255) / 256 < 148 * 8 ? (total + 255) / 256 : 148 * 8);
     if (dtype == SB_F32)
         sb::launch(bias_act_kernel<float>, dim3(blocks), dim3(256), 0, stream, (float*)out, (const float*)in, parts, S,
