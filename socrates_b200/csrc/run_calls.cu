@@ -25,7 +25,7 @@ int sb_attention_simt(void*, float*, float*, const void*, const void*, const voi
                       int, int, int, int, int, float, int, int, cudaStream_t);
 int sb_attention_prefill_tcgen05(void*, const void*, const void*, const void*, int, const int*, int, const int*, const int*,
                                  const int*, int, int, int, int, int, int, int, float, int*, const void*, long long, int, int,
-                                 float, int, float*, float, const float*, int, int, const float*, int, cudaStream_t);
+                                 float, int, float*, float, const float*, int, int, const float*, int, int, cudaStream_t);
 int sb_attention_prefill_mma(void*, const void*, const void*, const void*, const int*, int, const int*, const int*, const int*,
                              int, int, int, int, int, int, int, float, cudaStream_t);
 int sb_attention_balanced(void*, float*, float*, int*, const void*, const void*, const void*, const int*, int, const int*,

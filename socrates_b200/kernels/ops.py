@@ -540,7 +540,8 @@ def attention_prefill_tcgen05(out: torch.Tensor, q: torch.Tensor, k_pool: torch.
                               sink: Optional[float] = None, keep_first: int = 0,
                               out_float: Optional[torch.Tensor] = None, softcap: float = 0.0,
                               slopes: Optional[torch.Tensor] = None, chunk: int = 0,
-                              skip_single: bool = False, dist_bias: Optional[torch.Tensor] = None) -> None:
+                              skip_single: bool = False, dist_bias: Optional[torch.Tensor] = None,
+                              meta_older: bool = False) -> None:
     """Paged causal attention of prompt portions on tcgen05 (scores and P.V in tensor
     memory, pages brought in by TMA).  Arguments as `attention_prefill_mma`, plus the int32
     status word that receives a non-zero code if a bounded wait inside the kernel gave up.
@@ -548,7 +549,9 @@ def attention_prefill_tcgen05(out: torch.Tensor, q: torch.Tensor, k_pool: torch.
     [N, Hq*D]): the rows go there unrounded instead of to `out` (which may then be None).
     `softcap`, `slopes`, `chunk` as in `attention_decode_mma`.  `skip_single`: requests that bring one
     token are left out (see `attention_decode_balanced`); their rows of `out` are not written.  `dist_bias`
-    float32 [Hq, L]: joins the score of the key at distance min(d, L - 1), after the cap."""
+    float32 [Hq, L]: joins the score of the key at distance min(d, L - 1), after the cap.  `meta_older`: the block
+    table and the seq_ tensors are older than the kernel before this one on the stream (in a step they are: they
+    come with its one host copy), so they are read before that kernel has ended."""
     N = q.shape[0]
     pages, Hkv, BS, D = k_pool.shape
     R = seq_rows.numel()
@@ -581,7 +584,7 @@ def attention_prefill_tcgen05(out: torch.Tensor, q: torch.Tensor, k_pool: torch.
         _ptr(seq_starts), _ptr(seq_rows), _ptr(seq_first_pos), R, N, num_heads, Hkv, D, BS, int(window),
         float(scale), _ptr(status), _ptr(gate), gate_stride, int(gate_per_dim), int(sink is not None),
         float(sink or 0.0), int(keep_first), _ptr(out_float), float(softcap), _slopes(slopes, num_heads), int(chunk),
-        int(skip_single), _ptr(dist_bias), L, _stream()), "attention_prefill_tcgen05")
+        int(skip_single), _ptr(dist_bias), L, int(meta_older), _stream()), "attention_prefill_tcgen05")
 
 
 # ---------------------------------------------------------------------------------------------

@@ -105,7 +105,7 @@ def paged_attention(ctx, out, q, k_pool, v_pool, table, num_heads: int, scale: f
             apart = (paged_partition() is None and ctx.longest_single >= SINGLES_APART_FROM
                      and ops.attention_balanced_supports(num_heads, Hkv, D, page_size, ctx.num_seqs))
             ops.attention_prefill_tcgen05(out, q, k_pool, v_pool, table, ctx.seq_starts, ctx.seq_rows,
-                                          ctx.seq_first_pos, num_heads, scale, ctx.status, window, skip_single=apart)
+                                          ctx.seq_first_pos, num_heads, scale, ctx.status, window, skip_single=apart, meta_older=True)
             if apart:
                 balanced_attention(ctx, out, q, k_pool, v_pool, table, num_heads, scale, window)
             return

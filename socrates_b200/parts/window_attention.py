@@ -132,7 +132,7 @@ class WindowBiasAttention(Part):
                 and ops.attention_tcgen05_pages_supports(k_pool, table)):
             ops.attention_prefill_tcgen05(attn, q, k_pool, v_pool, table, ctx.seq_starts, ctx.seq_rows, ctx.seq_first_pos,
                                           self.H, self.scale, ctx.status, self.window or 0, gate=gate,
-                                          softcap=max(self.softcap, 0.0), dist_bias=self.dist_bias)
+                                          softcap=max(self.softcap, 0.0), dist_bias=self.dist_bias, meta_older=True)
             return Branch(self.o(ctx, attn, self.out_buffer, out="partial"))
         if portions and ops.attention_bias_tile_supports(self.H, self.G, self.dk, self.dv, ctx.dtype):
             # prompt portions: a tile of a request's consecutive tokens per block shares the keys it reads
