@@ -26,9 +26,22 @@ namespace {
 // half of every K block's products into an accumulator of its own (columns BN.. beside the
 // first), and the epilogue adds the two.  Where four such accumulators do not fit into the 512
 // columns, a tile's main loop waits for the epilogue of the tile before it.
+//
+// BN > 256 (always two issuers, one accumulator): a product is at most 256 columns wide, so one warp issues the first half of
+// the columns and the other the rest, and the W tile comes as two boxes.
+// Shared memory sets the pace (A is read once for each half), 0.475 us a K block at 288 columns for 0.36 at 256: they are for
+// products that then need one wave for two (pick_bn).
 constexpr int ACC_STRIDE = 256;          // TMEM columns between the two accumulators
 
-template <int BN, int ISSUERS> constexpr int acc_buffers() { return 2 * ISSUERS * BN <= 512 ? 2 : 1; }
+template <int BN, int ISSUERS> constexpr int acc_buffers() { return BN <= 256 && 2 * ISSUERS * BN <= 512 ? 2 : 1; }
+// columns of the first issuer's products (a multiple of 32), and rows of a box of W
+template <int BN> constexpr int first_columns() { return BN <= 256 ? BN : (BN / 2 + 31) / 32 * 32; }
+template <int BN> constexpr int w_box() { return BN <= 256 ? BN : BN / 2; }
+template <int BN>
+__device__ __forceinline__ void load_w_tile(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+    tma_load_2d(dst, map, bar, x, y);
+    if constexpr (BN > 256) tma_load_2d(dst + w_box<BN>() * BK * 2, map, bar, x, y + w_box<BN>());
+}
 
 template <int BN, int STAGES, typename TC, int EPI, int ISSUERS>
 __global__ void __launch_bounds__(160 + 32 * ISSUERS, 1)
@@ -85,7 +98,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const 
                 for (int i = 0; i < ahead; ++i) {
                     const uint32_t bar = smem_u32(&full_bar[i]);
                     mbar_arrive_expect_tx(bar, stage_bytes<BN>());
-                    tma_load_2d(tiles + i * stage_bytes<BN>() + BM * BK * 2, &tma_b, bar, i * BK, b0);
+                    load_w_tile<BN>(tiles + i * stage_bytes<BN>() + BM * BK * 2, &tma_b, bar, i * BK, b0);
                 }
                 sb::pdl_wait();
                 for (int i = 0; i < ahead; ++i)
@@ -98,7 +111,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const 
                     const uint32_t bar = smem_u32(&full_bar[s]);
                     mbar_arrive_expect_tx(bar, stage_bytes<BN>());
                     tma_load_2d(tiles + s * stage_bytes<BN>(), &tma_a, bar, i * BK, a0);
-                    tma_load_2d(tiles + s * stage_bytes<BN>() + BM * BK * 2, &tma_b, bar, i * BK, b0);
+                    load_w_tile<BN>(tiles + s * stage_bytes<BN>() + BM * BK * 2, &tma_b, bar, i * BK, b0);
                 }
                 continue;
             }
@@ -109,7 +122,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const 
                 const uint32_t bar = smem_u32(&full_bar[s]);
                 mbar_arrive_expect_tx(bar, stage_bytes<BN>());
                 tma_load_2d(tiles + s * stage_bytes<BN>(), &tma_a, bar, i * BK, a0);
-                tma_load_2d(tiles + s * stage_bytes<BN>() + BM * BK * 2, &tma_b, bar, i * BK, b0);
+                load_w_tile<BN>(tiles + s * stage_bytes<BN>() + BM * BK * 2, &tma_b, bar, i * BK, b0);
             }
         }
         if (!ok) {
@@ -121,10 +134,13 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const 
         }
     } else if (warp == 1 || warp == 6) {
         // ---------------- MMA issuer q (warp 1, and warp 6 when there are two)
-        constexpr uint32_t idesc = make_idesc(BN);
-        constexpr int NACC = acc_buffers<BN, ISSUERS>();
-        constexpr int KPER = (BK / UMMA_K) / ISSUERS;      // products of a K block per issuing thread
+        constexpr int NACC = acc_buffers<BN, ISSUERS>(), FIRST = first_columns<BN>();
+        constexpr bool BY_COLUMNS = BN > 256;              // the issuers share out the columns, not the K block
+        constexpr int KPER = (BK / UMMA_K) / (BY_COLUMNS ? 1 : ISSUERS);    // products of a K block per issuing thread
         const int q = warp == 1 ? 0 : 1;
+        const uint32_t idesc = BY_COLUMNS && q == 1 ? make_idesc(BN - FIRST) : make_idesc(FIRST);
+        const int a_step = BY_COLUMNS ? 0 : q * KPER * UMMA_K * 2;
+        const int b_step = BM * BK * 2 + (BY_COLUMNS ? q * FIRST * BK * 2 : a_step);
         uint32_t it = 0;
         int j = 0;                                         // tiles done by this block
         bool ok = true;
@@ -133,13 +149,13 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const 
             // the epilogue must have drained this accumulator (first use of each passes at once)
             if (j >= NACC && !mbar_wait_warp(smem_u32(&acc_empty[acc]), ((j / NACC) - 1) & 1)) { ok = false; break; }
             tcgen05_fence_after();
-            const uint32_t d = tmem_d + acc * ACC_STRIDE + q * BN;
+            const uint32_t d = tmem_d + acc * ACC_STRIDE + q * FIRST;
             for (int i = 0; i < kb_total; ++i, ++it) {
                 const int s = it % STAGES;
                 if (!mbar_wait_warp(smem_u32(&full_bar[s]), (it / STAGES) & 1)) { ok = false; break; }
                 tcgen05_fence_after();
-                const uint32_t sa = tiles + s * stage_bytes<BN>() + q * KPER * UMMA_K * 2;
-                const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + BM * BK * 2);
+                const uint32_t stage = tiles + s * stage_bytes<BN>();
+                const uint64_t da = make_smem_desc(stage + a_step), db = make_smem_desc(stage + b_step);
                 if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < KPER; ++k)          // the address is the low bits of a descriptor, in 16 bytes
@@ -177,10 +193,10 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const 
             if constexpr (sizeof(TC) == 4 && EPI == 0 && BN % 32 == 0) {
                 float* stage = reinterpret_cast<float*>(smem_raw + (tiles - smem_u32(smem_raw)) +
                                                         STAGES * stage_bytes<BN>() + quarter * kStageBytesPerWarp);
-                drain_tile_f32_staged<BN, (ISSUERS == 2 ? BN : 0)>(taddr, reinterpret_cast<float*>(C), M, N,
+                drain_tile_f32_staged<BN, (ISSUERS == 2 && BN <= 256 ? BN : 0)>(taddr, reinterpret_cast<float*>(C), M, N,
                                                                     a0 + quarter * 32, lane, b0, stage);
             } else {
-                drain_tile<BN, TC, EPI, (ISSUERS == 2 ? BN : 0)>(taddr, C, M, N, m, b0);
+                drain_tile<BN, TC, EPI, (ISSUERS == 2 && BN <= 256 ? BN : 0)>(taddr, C, M, N, m, b0);
             }
             tcgen05_fence_before();
             __syncwarp();
@@ -756,7 +772,7 @@ constexpr int pair_stages(int bn) {
 }
 
 // Tile widths of the persistent kernel, and the ring depth that fits in shared memory for each.
-#define SB_PERSISTENT_WIDTHS(X) X(256) X(160) X(128)
+#define SB_PERSISTENT_WIDTHS(X) X(256) X(160) X(128) X(288) X(352) X(416)
 constexpr int persistent_stages(int bn) {
     const int s = (222 * 1024 - kStageBytes) / (BM * BK * 2 + bn * BK * 2);
     return s > 6 ? 6 : s;
@@ -770,14 +786,19 @@ constexpr int persistent_stages(int bn) {
 // issued the products; with whole warps it is 598, 626 and 736 there, in the same proportions
 // within 5 %, and from 260 to 4,096 rows of the o and down projections of 4B, 8B and 32B the width
 // chosen is within 3 % of the fastest of the three.
+// Wider tiles (288 / 352 / 416 columns: 1,040 / 1,190 / 1,350 in the units below) where all are ONE wave, which has no epilogue
+// beside it, and eight row tiles or more share each panel of W: 2,048 x 2,560 x 9,728 80 us (160 columns 96, 256 115), x 4,096
+// 37 (45, 51), 1,024 x 6,144 x 2,560 30 (47, 38).  With two or three row tiles W's bytes set the pace and they lose: 187 x 19,456 x
+// 2,560 49 us (160 columns 45), 384 rows 64 (60).  A prompt of 1,023 tokens through 18 layers of 4B 5,287 -> 5,185 us.
 static int pick_bn(int M, int N, int num_sms) {
     const int tiles_m = (M + BM - 1) / BM;
     int best = 256;
     double best_cost = -1.0;
 #define SB_CONSIDER(bn) { \
         const long tiles = (long)tiles_m * ((N + bn - 1) / bn); \
-        const double cost = (double)((tiles + num_sms - 1) / num_sms) * (540.0 + 0.94 * bn); \
-        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = bn; } }
+        const long waves = (tiles + num_sms - 1) / num_sms; \
+        const double cost = (double)waves * (bn <= 256 ? 540.0 + 0.94 * bn : 340.0 + 2.42 * bn); \
+        if ((bn <= 256 || (waves == 1 && tiles_m >= 8)) && (best_cost < 0 || cost < best_cost)) { best_cost = cost; best = bn; } }
     SB_PERSISTENT_WIDTHS(SB_CONSIDER)
 #undef SB_CONSIDER
     return best;
@@ -788,7 +809,7 @@ static int pick_bn(int M, int N, int num_sms) {
 // heavier epilogue exposed, gate/up lost 4 %).  Taken again with issuing warps that walk their loops
 // whole, us with two / with one: 2,048 x 2,560 x 9,728 at width 160 96.9 / 98.1, at 128 139 / 143;
 // 512 rows 50.4 / 59.0 and 53.5 / 60.5; 1,999 x 5,120 x 25,600 604 / 612 and 724 / 762.
-constexpr int row_issuers(int bn, int epi) { return bn == 128 || (bn == 160 && epi == 0) ? 2 : 1; }
+constexpr int row_issuers(int bn, int epi) { return bn > 256 || bn == 128 || (bn == 160 && epi == 0) ? 2 : 1; }
 
 template <typename TC>
 int many_rows(const void* A, const void* W, void* C, int M, int N, int K, int* status, int variant, int epi,
@@ -819,8 +840,8 @@ int many_rows(const void* A, const void* W, void* C, int M, int N, int K, int* s
         int dev = 0, num_sms = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
-        const int bn = (variant >= 128 && variant <= 256 && variant % 16 == 0) ? variant : pick_bn(M, N, num_sms);
-        if (!get_map(&ma, A, M, K, BM) || !get_map(&mb, W, N, K, bn)) {
+        const int bn = (variant >= 128 && variant <= 256 && variant % 16 == 0) || variant == 288 || variant == 352 || variant == 416 ? variant : pick_bn(M, N, num_sms);
+        if (!get_map(&ma, A, M, K, BM) || !get_map(&mb, W, N, K, bn <= 256 ? bn : bn / 2)) {
             sb_set_error("gemm_tcgen05: cuTensorMapEncodeTiled failed (M=%d N=%d K=%d)", M, N, K);
             return SB_ERR_ARG;
         }
