@@ -169,6 +169,34 @@ template <int WARPS> __device__ __forceinline__ float block_sum_once(float v, fl
     return t;
 }
 
+// block_sum of a block of G * 32 * WARPS threads, in its order of additions, by 32 * WARPS threads with one barrier: v[g] is
+// what thread threadIdx.x + 32 * WARPS * g of that block would bring.  `slot`: G * WARPS (at most 32) floats of shared memory
+// that nothing else uses.  warp_sum's tree for all g at once: as long as there are several values a lane, a shuffle halves them.
+template <int G, int WARPS> __device__ __forceinline__ float block_sum_as(const float (&v)[G], float* slot) {
+    static_assert(G <= 8 && G * WARPS <= 32, "one warp adds the warps' sums");
+    constexpr int P = G > 4 ? 8 : G > 2 ? 4 : G;
+    const int lane = threadIdx.x & 31;
+    float a[P];
+#pragma unroll
+    for (int g = 0; g < P; ++g) a[g] = g < G ? v[g] : 0.f;
+    int o = 16;
+#pragma unroll
+    for (int n = P / 2; n > 0; n /= 2, o /= 2) {
+        const bool upper = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float keep = upper ? a[i + n] : a[i], send = upper ? a[i] : a[i + n];
+            a[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+#pragma unroll
+    for (; o > 0; o /= 2) a[0] += __shfl_xor_sync(0xffffffffu, a[0], o);
+    const int g = lane / (32 / P);                          // whose sum this lane ends with
+    if (lane % (32 / P) == 0 && g < G) slot[g * WARPS + (threadIdx.x >> 5)] = a[0];
+    __syncthreads();
+    return warp_sum(lane < G * WARPS ? slot[lane] : 0.f);
+}
+
 // 4 floats to 4 elements of T, aligned to their size.
 __device__ __forceinline__ void store_four(float* p, float a, float b, float c, float d) {
     *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);

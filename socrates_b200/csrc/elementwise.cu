@@ -202,13 +202,16 @@ __global__ void __launch_bounds__(DEPTH > 8 ? 640 : 768) add_rmsnorm_vec_kernel(
 // With a column or three a thread, the row in shared memory and block_sum's barriers / so (us): 2,048 rows of 2,560 with two
 // parts (94 MB) 25.0 / 15.0, with one 15.6 / 12.3, 5,120 wide with two 43.0 / 29.2; 1,000 rows of 4,096 with one 13.6 / 10.1; 187 of
 // 2,560 with one 3.9 / 2.9, 65 2.5 / 2.5.
-template <typename T, int V, int THR>
+// A row's squares are added in the order of the kernel above with ORDER threads (a thread here stands for those THR apart), so a
+// row has the bits that it has there.
+template <typename T, int V, int THR, int ORDER>
 __global__ void __launch_bounds__(THR) add_rmsnorm_rows_kernel(float* __restrict__ residual, const float* __restrict__ delta, int S,
                                                                size_t delta_stride, const float* __restrict__ gain,
                                                                T* __restrict__ out, const int* __restrict__ row_index, int d,
                                                                float eps, int write_residual) {
     sb::pdl_launch_dependents();
-    __shared__ float slot[THR / 32];
+    constexpr int STANDS = ORDER / THR < V ? ORDER / THR : V;       // threads of the other kernel that one here stands for
+    __shared__ float slot[STANDS * THR / 32];
     const int m = blockIdx.x, d4 = d / 4, tid = threadIdx.x;
     sb::pdl_wait();
     const int r = row_index ? row_index[m] : m;
@@ -242,14 +245,14 @@ __global__ void __launch_bounds__(THR) add_rmsnorm_rows_kernel(float* __restrict
 #pragma unroll
         for (int c = 0; c < V; ++c) add4(v[c], p[c]);
     }
-    float ss = 0.f;
+    float ss[STANDS] = {};
 #pragma unroll
     for (int c = 0; c < V; ++c) {
         const int i = tid + c * THR;
         if (write_residual && i < d4) res4[i] = v[c];
-        if (i < d4) ss += squares4(v[c]);
+        if (i < d4) ss[c % STANDS] += squares4(v[c]);
     }
-    const float rinv = 1.0f / sqrtf(block_sum_once<THR / 32>(ss, slot) / (float)d + eps);
+    const float rinv = 1.0f / sqrtf(block_sum_as<STANDS, THR / 32>(ss, slot) / (float)d + eps);
     const float4* gain4 = reinterpret_cast<const float4*>(gain);
     T* o = out + (size_t)m * d;
 #pragma unroll
@@ -261,11 +264,13 @@ __global__ void __launch_bounds__(THR) add_rmsnorm_rows_kernel(float* __restrict
     }
 }
 
-// V and THR for a row of d4 columns; false: it is too wide for registers.
+// V and THR for a row of d4 columns (ORDER: the threads that sb_add_rmsnorm gives the kernel above for as many rows); false: it
+// is too wide for registers.
 template <typename T, typename... Args> bool launch_norm_rows(int M, int d4, cudaStream_t stream, Args... args) {
 #define SB_ROWS(V_, THR_)                                                                                                \
     if (d4 <= V_ * THR_) {                                                                                               \
-        sb::launch(add_rmsnorm_rows_kernel<T, V_, THR_>, dim3(M), dim3(THR_), 0, stream, args...);                         \
+        if (M > 512) sb::launch(add_rmsnorm_rows_kernel<T, V_, THR_, 256>, dim3(M), dim3(THR_), 0, stream, args...);       \
+        else sb::launch(add_rmsnorm_rows_kernel<T, V_, THR_, 768>, dim3(M), dim3(THR_), 0, stream, args...);               \
         return true;                                                                                                     \
     }
     SB_ROWS(2, 128) SB_ROWS(4, 128) SB_ROWS(5, 128) SB_ROWS(6, 128) SB_ROWS(4, 256) SB_ROWS(5, 256) SB_ROWS(6, 256) SB_ROWS(8, 256)
@@ -292,7 +297,7 @@ extern "C" int sb_add_rmsnorm(float* residual, const float* delta, int S, long l
     // regime, where the S partial sums of a column should all be in flight at once; so are 65 to 256
     // rows behind a product in many parts)
     const bool deep = M <= 64 || (M <= 256 && S > 2);
-    // many rows: in registers.  (Float32 rows keep the kernels of few rows, for the order of a row's squares.)
+    // many rows: in registers.  (Rows of float32 results keep the kernel above.)
     if (vec && !deep && dtype == SB_BF16 &&
         launch_norm_rows<__nv_bfloat16>(M, d / 4, stream, residual, delta, S, (size_t)delta_stride, gain, (__nv_bfloat16*)out,
                                         row_index, d, eps, write_residual))

@@ -241,6 +241,16 @@ template <int V, int THR> __device__ __forceinline__ float squares(const float4 
         if (threadIdx.x + c * THR < d4) ss += squares4(b[c]);
     return ss;
 }
+// The row's sum of squares in the order of fold_rmsnorm_vec_kernel with ORDER threads (block_sum_as).
+template <int ORDER, int V, int THR> constexpr int stands_for() { return ORDER / THR < V ? ORDER / THR : V; }
+template <int ORDER, int V, int THR> __device__ __forceinline__ float row_squares(const float4 (&b)[V], int d4, float* slot) {
+    constexpr int STANDS = stands_for<ORDER, V, THR>();
+    float ss[STANDS] = {};
+#pragma unroll
+    for (int c = 0; c < V; ++c)
+        if (threadIdx.x + c * THR < d4) ss[c % STANDS] += squares4(b[c]);
+    return block_sum_as<STANDS, THR / 32>(ss, slot);
+}
 // v[c] <- f(v[c], the column's float4 of t) for the columns there are
 template <int V, int THR, typename F> __device__ __forceinline__ void with_columns(float4 (&v)[V], const float* t, int d4, F f) {
     const float4* t4 = reinterpret_cast<const float4*>(t);
@@ -255,11 +265,11 @@ template <int V, int THR, typename F> __device__ __forceinline__ void with_colum
 // its way while the branch is normed and one barrier a sum (above, the row goes through shared memory and the residual is
 // loaded after the branch's norm).
 // The kernel above / this one (us), two parts with a gain: 2,048 rows of 2,048 39.7 / 16.2, 1,500 31.9 / 12.9, 300 9.6 / 4.3, 65
-// 4.1 / 3.7.
-template <typename T, int V, int THR>
+// 4.1 / 3.7.  The squares are added in the order of the kernel above with ORDER threads, so a row has the bits that it has there.
+template <typename T, int V, int THR, int ORDER>
 __global__ void __launch_bounds__(THR) fold_rmsnorm_rows_kernel(FoldArgs a) {
     sb::pdl_launch_dependents();
-    __shared__ float slot[2][THR / 32];
+    __shared__ float slot[2][stands_for<ORDER, V, THR>() * THR / 32];
     const int m = blockIdx.x, d4 = a.d / 4, tid = threadIdx.x;
     sb::pdl_wait();
     const int r = a.row_index ? a.row_index[m] : m;
@@ -272,7 +282,7 @@ __global__ void __launch_bounds__(THR) fold_rmsnorm_rows_kernel(FoldArgs a) {
         sum_parts<V, THR, 2>(b, a.delta, a.S, a.delta_stride, r, d4);
         if (a.branch_bias) with_columns<V, THR>(b, a.branch_bias, d4, [](float4& u, const float4& t) { add4(u, t); });
         if (a.branch_gain) {
-            const float binv = 1.0f / sqrtf(block_sum_once<THR / 32>(squares<V, THR>(b, d4), slot[0]) / (float)a.d + a.branch_eps);
+            const float binv = 1.0f / sqrtf(row_squares<ORDER, V, THR>(b, d4, slot[0]) / (float)a.d + a.branch_eps);
             with_columns<V, THR>(b, a.branch_gain, d4, [&](float4& u, const float4& t) {
                 u.x *= binv * t.x; u.y *= binv * t.y; u.z *= binv * t.z; u.w *= binv * t.w;
             });
@@ -293,7 +303,7 @@ __global__ void __launch_bounds__(THR) fold_rmsnorm_rows_kernel(FoldArgs a) {
     if (a.out == nullptr && !a.norm_residual) return;
     const bool squash = a.tanh_alpha != nullptr, normed = a.gain != nullptr && !squash;
     const float alpha = squash ? *a.tanh_alpha : 0.f;
-    const float rinv = normed ? 1.0f / sqrtf(block_sum_once<THR / 32>(squares<V, THR>(v, d4), slot[1]) / (float)a.d + a.eps) : 1.0f;
+    const float rinv = normed ? 1.0f / sqrtf(row_squares<ORDER, V, THR>(v, d4, slot[1]) / (float)a.d + a.eps) : 1.0f;
     T* o = (T*)a.out + (size_t)m * a.d;
 #pragma unroll
     for (int c = 0; c < V; ++c) {
@@ -493,10 +503,12 @@ extern "C" int sb_fold_rmsnorm(float* residual, const float* delta, int S, long 
     const bool vec = d % 4 == 0 && delta_stride % 4 == 0 && aligned(residual) && aligned(delta) && aligned(branch_bias) &&
                      aligned(branch_gain) && aligned(add_rows) && aligned(add_vec) && aligned(gain) && aligned(tanh_bias) &&
                      aligned(out);
-    // many rows of few parts: in registers.  (Few rows want every part of a column in flight; float32 rows keep to the one
-    // kernel in any batch, for the order of their squares.)
+    // many rows of few parts: in registers.  (Few rows want every part of a column in flight; rows of float32 results keep
+    // the kernel below.  ORDER: the threads that it takes for as many rows.)
     if (vec && M > 64 && S <= 4 && out_dtype == SB_BF16 && d <= 8192) {
-#define SB_FOLD(V_, THR_) sb::launch(fold_rmsnorm_rows_kernel<__nv_bfloat16, V_, THR_>, dim3(M), dim3(THR_), 0, stream, a)
+#define SB_FOLD(V_, THR_)                                                                                                \
+        if (M > 512) sb::launch(fold_rmsnorm_rows_kernel<__nv_bfloat16, V_, THR_, 256>, dim3(M), dim3(THR_), 0, stream, a);  \
+        else sb::launch(fold_rmsnorm_rows_kernel<__nv_bfloat16, V_, THR_, 512>, dim3(M), dim3(THR_), 0, stream, a)
         SB_FOR_ROWS(d / 4, SB_FOLD);
 #undef SB_FOLD
         SB_LAUNCH_CHECK();

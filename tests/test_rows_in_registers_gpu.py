@@ -101,3 +101,34 @@ def test_bias_act(ops, dtype, act, S):
         ops.bias_act(out, x, bias, act)
         outs.append(out.clone())
     assert torch.equal(*outs) and bool(torch.isfinite(outs[0]).all())
+
+
+@pytest.mark.parametrize("d", [4, 516, 1024, 2048, 2560, 3076, 4096, 5120, 8192])
+@pytest.mark.parametrize("M,S", [(65, 2), (300, 0), (512, 1), (513, 2), (900, 3)])
+def test_add_rmsnorm_rows_have_the_other_kernels_bits(ops, d, M, S):
+    """float32 results come from the kernel with a row in shared memory: the same numbers, rounded once more."""
+    g = torch.Generator(device=DEV).manual_seed(d * M + S)
+    res, gain = torch.randn(M, d, device=DEV, generator=g), torch.randn(d, device=DEV, generator=g)
+    delta = torch.randn(S, M, d, device=DEV, generator=g) if S else None
+    sides = []
+    for dtype in (torch.bfloat16, torch.float32):
+        r, out = res.clone(), torch.full((M, d), float("nan"), device=DEV, dtype=dtype)
+        ops.add_rmsnorm(r, delta, gain, out, EPS)
+        sides.append((r, out.to(torch.bfloat16)))
+    assert torch.equal(sides[0][0], sides[1][0]) and torch.equal(sides[0][1], sides[1][1])
+
+
+@pytest.mark.parametrize("d", [8, 1024, 2052, 2560, 4096, 8192])
+@pytest.mark.parametrize("M", [65, 512, 513])
+@pytest.mark.parametrize("form", ["plain", "normed", "norm_residual"])
+def test_fold_rmsnorm_rows_have_the_other_kernels_bits(ops, d, M, form):
+    g = torch.Generator(device=DEV).manual_seed(d + M)
+    res, delta = torch.randn(M, d, device=DEV, generator=g), torch.randn(3, M, d, device=DEV, generator=g)
+    gain, inner = torch.randn(d, device=DEV, generator=g), torch.randn(d, device=DEV, generator=g)
+    kw = {"normed": dict(branch_gain=inner, branch_eps=EPS), "norm_residual": dict(norm_residual=True)}.get(form, {})
+    sides = []
+    for dtype in (torch.bfloat16, torch.float32):
+        r, out = res.clone(), torch.full((M, d), float("nan"), device=DEV, dtype=dtype)
+        ops.fold_rmsnorm(r, delta, gain, out, EPS, **kw)
+        sides.append((r, out.to(torch.bfloat16)))
+    assert torch.equal(sides[0][0], sides[1][0]) and torch.equal(sides[0][1], sides[1][1])
