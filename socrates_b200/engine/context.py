@@ -157,12 +157,16 @@ class StepContext:
             parts = self.wide_splits(M, w, x_dtype)
             if parts:
                 return parts
-            parts = self.gemm_shares(M, w, x_dtype) if shares else 0
-            if parts:
-                return parts
+            served = self._shares_parts(M, w, x_dtype) if shares else 0
+            if served and self._shares_pay(M, w):
+                return served
             # Many rows but few tiles (a short prompt portion through a narrow projection): cut K
             # so that the tiles cover the SMs.  Measured on the 4B shape at 512 rows: o 29 -> 20 us,
             # down 57 -> 33 us with three parts; from 1,024 rows on a cut no longer pays.
+            # Where equal shares serve the shape and were refused, they were refused for whole tiles, and a cut in two is no
+            # better than those: with the norm that adds the parts, equal shares / cut in two / whole tiles (us): 2,560 x
+            # 4,096: 513 rows 33.5 / 28.7 / 22.8, 896 41.2 / 31.0 / 25.1; 2,560 x 9,728: 640 49.4 / 47.4 / 43.0; 4,096 x 4,096:
+            # 450 33.8 / 26.1 / 24.3; 5,120 x 8,192: 384 51.5 / 46.3 / 41.7; in three 4,096 x 4,096: 300 31.7 / 22.5 / 23.8.
             # The cut is kept to the regime it was measured in.  Beyond it the one-tile-per-block kernel has
             # stalled: 2,048 rows through a 1,024 x 16,384 matrix cut in two (all experts' down matrices side
             # by side) never came back in about one first step in five, with every wait inside it bounded;
@@ -170,7 +174,8 @@ class StepContext:
             tiles = -(-M // 128) * -(-N // 256)
             if 2 * tiles > self.num_sms or M >= 1024:
                 return 1
-            return ops.gemm_tcgen05_splits(K, max(1, min(4, self.num_sms // tiles, (-(-K // 64)) // 8)))
+            parts = ops.gemm_tcgen05_splits(K, max(1, min(4, self.num_sms // tiles, (-(-K // 64)) // 8)))
+            return 1 if served and parts == 2 else parts
         tiles = -(-N // 128)
         want = max(1, (2 * self.num_sms) // tiles)
         most = max(1, (-(-K // 64)) // 2)
@@ -205,6 +210,14 @@ class StepContext:
             return 0
         return ops.gemm_tcgen05_splits(K, parts)
 
+    def _shares_parts(self, M: int, w: torch.Tensor, x_dtype: torch.dtype) -> int:
+        """Parts that the pair kernel in equal shares of K blocks writes for a product of M rows; 0: it does not serve the
+        shape, or both operands together are more than the 96 MB that stay well inside the L2 cache (see gemm_shares)."""
+        if not self.uses_tensor_cores(x_dtype, w) or os.environ.get("SOCRATES_GEMM_SHARES", "1") == "0":
+            return 0
+        N, K = w.shape
+        return 0 if (M + N) * K * 2 > 96 * (1 << 20) else ops.gemm_tcgen05_shares_parts(M, N, K)
+
     def gemm_shares(self, M: int, w: torch.Tensor, x_dtype: torch.dtype) -> int:
         """Parts of the pair kernel in equal shares of K blocks if a product of M rows whose output
         is partial sums should run on it, else 0.  Whole tiles run in waves over the SMs; a product
@@ -223,14 +236,12 @@ class StepContext:
         1,280 58.7 / 62.2, 1,500 71.3 / 63.2, 2,048 89.1 / 98.6; 2,560 x 4,096: 1,023 32.3 / 21.0, 2,048 45.4 / 44.9; 4,096 x 4,096:
         512 26.5 / 19.8, 1,023 36.9 / 29.7, 1,280 42.1 / 44.9, 1,500 47.6 / 52.2, 1,792 53.3 / 52.6; 5,120 x 8,192: 512 48.1 / 41.9,
         1,023 74.4 / 85.3."""
-        if not self.uses_tensor_cores(x_dtype, w) or os.environ.get("SOCRATES_GEMM_SHARES", "1") == "0":
-            return 0
+        parts = self._shares_parts(M, w, x_dtype)
+        return parts if parts and self._shares_pay(M, w) else 0
+
+    def _shares_pay(self, M: int, w: torch.Tensor) -> bool:
+        """gemm_shares' costs."""
         N, K = w.shape
-        if (M + N) * K * 2 > 96 * (1 << 20):
-            return 0
-        parts = ops.gemm_tcgen05_shares_parts(M, N, K)
-        if parts == 0:
-            return 0
         pairs = max(1, self.num_sms // 2)
         kb, rows128 = -(-K // 64), -(-M // 128)
         shares_cost = 13.9 + 0.455 * kb * -(-M // 256) * -(-N // 256) / pairs
@@ -241,7 +252,7 @@ class StepContext:
                          for bn, one, more in ((128, 0.215, 0.27), (160, 0.26, 0.297), (256, 0.365, 0.357)))
         if M >= 4096:       # the pair kernel with whole tiles is the choice there
             whole_cost = min(whole_cost, whole(-(-(-(-M // 256) * -(-N // 256)) // pairs), 0.34, 0.34))
-        return parts if shares_cost < 1.02 * whole_cost else 0
+        return shares_cost < 1.02 * whole_cost
 
     def can_fuse_silu_mul(self, M: int, w: torch.Tensor, x_dtype: torch.dtype) -> bool:
         """Whether the product with an interleaved gate/up matrix can apply the gated unit (SiLU or gelu) in its
