@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(256) short_conv_kernel(ConvArgs a) {
 
 // The same for many tokens: a thread holds 16 bytes of neighbouring channels (VEC) and walks RUN tokens of the batch with the
 // last K - 1 values in registers, so that a value is read once and not K times, in whole lines.  The sums are those of the
-// kernel above, in its order.  A prompt of 1,500 tokens through 3,072 channels of 3 taps and 4,096 of 4, twice each: 237 us with a
+// kernel above, in its order (which call takes which: sb_short_conv_pays_runs).  A prompt of 1,500 tokens through 3,072 channels of 3 taps and 4,096 of 4, twice each: 237 us with a
 // thread a value, 102 here.
 constexpr int RUN = 8;
 
@@ -250,13 +250,27 @@ __global__ void __launch_bounds__(256) short_conv_tail_kernel(float* __restrict_
 
 }  // namespace
 
-// seg_*: arrays of `nseg` entries describing the destinations (see ConvSeg).
+// Whether N tokens of `requests` requests by C channels of K taps go by runs (short_conv_runs_kernel) where their layout allows
+// it (1) or a value a thread (0).  A run is eight tokens one after another, 9 to 14 us whatever their number, and more where a
+// run meets many requests (each starts with a round trip for its row and one for its tail); a thread a value takes a time in
+// proportion to the values.  Runs / a thread a value (us), by millions (2^20) of values: 4 taps in bfloat16, one portion: 0.75
+// 10.9 / 9.7, 1.0 11.4 / 12.4, 2.0 12.0 / 22.8; decoding requests: 0.25 12.9 / 4.7 (64 through 4,096 channels), 1.0 14.3 / 12.0,
+// 1.25 14.6 / 14.4, 1.5 14.7 / 16.9; one decoding request in eight tokens: 1.0 13.8 / 12.3, 1.25 13.9 / 14.9; 2 taps, decoding:
+// 1.25 11.8 / 10.8, 1.5 11.9 / 12.5.  float32, 4 taps: one portion 0.5 6.7 / 7.1; decoding 0.75 9.7 / 9.4, 1.0 9.9 / 11.8.
+extern "C" int sb_short_conv_pays_runs(int N, int C, int K, int requests, int dtype) {
+    long long least = requests <= 2 ? (dtype == SB_BF16 ? 1 << 20 : 1 << 19) : (dtype == SB_BF16 ? 5 << 18 : 7 << 17);
+    if (K == 2) least += least / 4;
+    return (long long)N * C >= least;
+}
+
+// seg_*: arrays of `nseg` entries describing the destinations (see ConvSeg).  `requests`: how many the tokens are of (for the
+// choice of the kernel alone; as many as tokens where it is not known).
 extern "C" int sb_short_conv(const void* in, long long in_stride, const float* in_bias, const float* taps,
                              const float* conv_bias, int act, const float* tail, int C, int K, int N,
                              const int* token_rows, const int* positions, const int* block_table,
                              int table_width, int page_size, int nseg, const int* seg_begin, const int* seg_end,
                              const int* seg_paged, void* const* seg_dst, const long long* seg_stride,
-                             const int* seg_heads, const int* seg_head_dim, int dtype, cudaStream_t stream) {
+                             const int* seg_heads, const int* seg_head_dim, int requests, int dtype, cudaStream_t stream) {
     SB_REQUIRE(C > 0 && N >= 0 && K >= 1 && K <= MAX_TAPS, "short_conv: bad sizes C=%d N=%d taps=%d (at most %d)", C, N, K,
                MAX_TAPS);
     SB_REQUIRE(nseg >= 1 && nseg <= 3, "short_conv: %d destinations (1 to 3)", nseg);
@@ -274,8 +288,8 @@ extern "C" int sb_short_conv(const void* in, long long in_stride, const float* i
         SB_REQUIRE(!a.seg[s].paged || (block_table != nullptr && page_size > 0 && a.seg[s].head_dim > 0),
                    "short_conv: a paged destination needs a block table");
     }
-    // from 64 tokens on (a decode step's few tokens are all first of their request, where a run saves nothing)
-    if (N >= 64 && ((dtype == SB_F32 && runs_take<float>(a)) || (dtype == SB_BF16 && runs_take<__nv_bfloat16>(a)))) {
+    if (sb_short_conv_pays_runs(N, C, K, requests, dtype) &&
+        ((dtype == SB_F32 && runs_take<float>(a)) || (dtype == SB_BF16 && runs_take<__nv_bfloat16>(a)))) {
         if (dtype == SB_F32) launch_runs<float>(a, stream);
         else launch_runs<__nv_bfloat16>(a, stream);
         SB_LAUNCH_CHECK();

@@ -680,13 +680,14 @@ def bias_act(out: torch.Tensor, x: torch.Tensor, bias: Optional[torch.Tensor], a
 def short_conv(x: torch.Tensor, in_bias: Optional[torch.Tensor], taps: torch.Tensor,
                conv_bias: Optional[torch.Tensor], silu: bool, tail: Optional[torch.Tensor],
                token_rows: torch.Tensor, positions: torch.Tensor, destinations,
-               block_table: Optional[torch.Tensor] = None) -> None:
+               block_table: Optional[torch.Tensor] = None, requests: Optional[int] = None) -> None:
     """Causal convolution over time of the first C columns of x [N, >= C], per channel.
 
     y_t = act(sum_j taps[:, j] * (x + in_bias)_{t-K+1+j} + conv_bias), zeros before a sequence's start; tokens
     before the step's portion come from `tail` float32 [rows, K-1, C] (not changed here: `short_conv_tail`).
     `destinations`: up to three (begin, end, tensor) column ranges; a 2-d tensor [N, end-begin] is written
     densely, a 4-d pool [pages, heads, page_size, head_dim] at each token's slot through `block_table`.
+    `requests`: how many the tokens are of, where the caller knows it (the kernel is chosen by it, the results are the same).
     """
     C, K = taps.shape
     N = x.shape[0]
@@ -732,7 +733,13 @@ def short_conv(x: torch.Tensor, in_bias: Optional[torch.Tensor], taps: torch.Ten
     check(lib, lib.sb_short_conv(_ptr(x), x.stride(0), _ptr(in_bias), _ptr(taps), _ptr(conv_bias), int(silu),
                                  _ptr(tail), C, K, N, _ptr(token_rows), _ptr(positions), _ptr(block_table),
                                  block_table.shape[1] if block_table is not None else 0, page_size, n, begin, end,
-                                 paged, dst, stride, heads, hd, _code(x.dtype), _stream()), "short_conv")
+                                 paged, dst, stride, heads, hd, N if requests is None else int(requests), _code(x.dtype),
+                                 _stream()), "short_conv")
+
+
+def short_conv_pays_runs(N: int, C: int, K: int, requests: int, dtype: torch.dtype) -> bool:
+    """Whether `short_conv` walks N tokens of `requests` requests in runs (where the layout allows it)."""
+    return bool(library().sb_short_conv_pays_runs(N, C, K, requests, _code(dtype)))
 
 
 def short_conv_tail(tail: torch.Tensor, x: torch.Tensor, in_bias: Optional[torch.Tensor], taps: int,

@@ -89,7 +89,8 @@ class GatedDeltaRule(Part):
         proj = self.proj(ctx, x, "dr_proj")
         conv = ctx.buffers.take("dr_conv", N, (C,), ctx.dtype)
         tail = cache.state("conv") if self.taps > 1 else None
-        ops.short_conv(proj, None, self.conv, None, True, tail, ctx.token_rows, ctx.positions, [(0, C, conv)])
+        ops.short_conv(proj, None, self.conv, None, True, tail, ctx.token_rows, ctx.positions, [(0, C, conv)],
+                       requests=ctx.num_seqs)
         if tail is not None:
             ops.short_conv_tail(tail, proj, None, self.taps, ctx.seq_starts, ctx.seq_rows)
         y = ctx.buffers.take("dr_y", N, (self.Cv,), ctx.dtype)

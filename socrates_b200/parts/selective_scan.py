@@ -77,7 +77,8 @@ class SelectiveScan(Part):
         xz = self.w_in(ctx, x, "ss_xz")
         xc = ctx.buffers.take("ss_x", N, (I,), ctx.dtype)
         tail = cache.state("conv") if self.taps > 1 else None
-        ops.short_conv(xz, None, self.conv, self.conv_bias, True, tail, ctx.token_rows, ctx.positions, [(0, I, xc)])
+        ops.short_conv(xz, None, self.conv, self.conv_bias, True, tail, ctx.token_rows, ctx.positions, [(0, I, xc)],
+                       requests=ctx.num_seqs)
         if tail is not None:
             ops.short_conv_tail(tail, xz, None, self.taps, ctx.seq_starts, ctx.seq_rows)
         dt_in = self.w_dtin(ctx, xc, "ss_dtin")

@@ -1,5 +1,5 @@
-"""The convolution's kernel for many tokens: the same bits as the kernel for few, which serves the same tokens in steps of fewer
-than 64 and any call that has no whole 16-byte pieces."""
+"""The convolution's kernel for many values: the same bits as the kernel for few, which serves smaller steps and any call that has
+no whole 16-byte pieces."""
 
 import pytest
 import torch
@@ -59,3 +59,43 @@ def test_runs(ops, dtype, K, bias, silu):
         # K + 2 float32 roundings, the gate's few, and the result's own
         bound = (K + 12) * 2.0 ** -24 * (mag + acc.abs() + 10) + (2.0 ** -8 * acc.abs() if dtype == torch.bfloat16 else 0)
         assert bool(((runs[0][n].double() - acc).abs() <= bound).all()), n
+
+
+@pytest.mark.parametrize("N,C,K,requests,dtype,runs", [
+    (64, 3072, 3, 64, torch.bfloat16, False), (64, 4096, 4, 64, torch.bfloat16, False), (256, 4096, 4, 256, torch.bfloat16, False),
+    (319, 4096, 4, 3, torch.bfloat16, False), (320, 4096, 4, 320, torch.bfloat16, True), (187, 4096, 4, 1, torch.bfloat16, False),
+    (255, 4096, 4, 1, torch.bfloat16, False), (256, 4096, 4, 2, torch.bfloat16, True), (1500, 3072, 3, 1, torch.bfloat16, True),
+    (64, 4096, 4, 64, torch.float32, False), (128, 4096, 4, 1, torch.float32, True), (223, 4096, 4, 223, torch.float32, False),
+    (224, 4096, 4, 224, torch.float32, True), (191, 8192, 2, 191, torch.bfloat16, False), (200, 8192, 2, 200, torch.bfloat16, True)])
+def test_which_steps_go_by_runs(ops, N, C, K, requests, dtype, runs):
+    assert ops.short_conv_pays_runs(N, C, K, requests, dtype) == runs
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("K", [2, 3, 4])
+@pytest.mark.parametrize("lengths", [(1,) * 420, (331,), (300, 1, 9, 1, 2, 100)])
+def test_wide_rows_by_runs(ops, dtype, K, lengths):
+    """Enough values for runs: the same bits as a thread a value (taps off 16 bytes), dense and paged, and with a step that
+    does not say how many requests it is of."""
+    heads, dim, page, N, R = 8, 64, 16, sum(lengths), len(lengths)
+    dense = 4608
+    C = dense + heads * dim
+    g = torch.Generator(device=DEV).manual_seed(K)
+    assert ops.short_conv_pays_runs(N, C, K, R, dtype)
+    x = torch.randn(N, C + 8, device=DEV, generator=g).to(dtype)
+    taps, tail = torch.randn(C, K, device=DEV, generator=g), torch.randn(R, K - 1, C, device=DEV, generator=g)
+    token_rows = torch.tensor([r for r, n in enumerate(lengths) for _ in range(n)], dtype=torch.int32, device=DEV)
+    positions = torch.tensor([r % 5 + i for r, n in enumerate(lengths) for i in range(n)], dtype=torch.int32, device=DEV)
+    pages = -(-(max(lengths) + 5) // page)
+    table = torch.arange(1, R * pages + 1, dtype=torch.int32, device=DEV).view(R, pages)
+    outs = []
+    for shift, requests in ((0, R), (0, None), (1, R)):
+        t = torch.empty(taps.numel() + shift, device=DEV)[shift:].view(taps.shape).copy_(taps)
+        out = torch.full((N, dense), float("nan"), device=DEV, dtype=dtype)
+        pool = torch.full((R * pages + 1, heads, page, dim), 7.0, device=DEV, dtype=dtype)
+        ops.short_conv(x, None, t, None, True, tail, token_rows, positions, [(0, dense, out), (dense, C, pool)], table,
+                       requests=requests)
+        outs.append((out, pool))
+    for out, pool in outs[1:]:
+        assert torch.equal(out, outs[0][0]) and torch.equal(pool, outs[0][1])
+    assert bool(torch.isfinite(outs[0][0]).all())
