@@ -171,7 +171,7 @@ template <int WARPS> __device__ __forceinline__ float block_sum_once(float v, fl
 
 // block_sum of a block of G * 32 * WARPS threads, in its order of additions, by 32 * WARPS threads with one barrier: v[g] is
 // what thread threadIdx.x + 32 * WARPS * g of that block would bring.  `slot`: G * WARPS (at most 32) floats of shared memory
-// that nothing else uses.  warp_sum's tree for all g at once: as long as there are several values a lane, a shuffle halves them.
+// that nothing else uses, on 16 bytes.  warp_sum's tree for all g at once: as long as there are several values a lane, a shuffle halves them.
 template <int G, int WARPS> __device__ __forceinline__ float block_sum_as(const float (&v)[G], float* slot) {
     static_assert(G <= 8 && G * WARPS <= 32, "one warp adds the warps' sums");
     constexpr int P = G > 4 ? 8 : G > 2 ? 4 : G;
@@ -194,7 +194,20 @@ template <int G, int WARPS> __device__ __forceinline__ float block_sum_as(const 
     const int g = lane / (32 / P);                          // whose sum this lane ends with
     if (lane % (32 / P) == 0 && g < G) slot[g * WARPS + (threadIdx.x >> 5)] = a[0];
     __syncthreads();
-    return warp_sum(lane < G * WARPS ? slot[lane] : 0.f);
+    constexpr int SLOTS = G * WARPS;
+    if constexpr (SLOTS <= 16) {                            // the tree of a warp's lanes, by every thread
+        constexpr int N = SLOTS <= 4 ? 4 : SLOTS <= 8 ? 8 : 16;
+        float t[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) t[i] = i < SLOTS ? slot[i] : 0.f;
+#pragma unroll
+        for (int n = N / 2; n > 0; n /= 2)
+#pragma unroll
+            for (int i = 0; i < n; ++i) t[i] += t[i + n];
+        return t[0];
+    } else {
+        return warp_sum(lane < SLOTS ? slot[lane] : 0.f);
+    }
 }
 
 // 4 floats to 4 elements of T, aligned to their size.

@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(THR) add_rmsnorm_rows_kernel(float* __restrict
                                                                float eps, int write_residual) {
     sb::pdl_launch_dependents();
     constexpr int STANDS = ORDER / THR < V ? ORDER / THR : V;       // threads of the other kernel that one here stands for
-    __shared__ float slot[STANDS * THR / 32];
+    __shared__ __align__(16) float slot[STANDS * THR / 32];
     const int m = blockIdx.x, d4 = d / 4, tid = threadIdx.x;
     sb::pdl_wait();
     const int r = row_index ? row_index[m] : m;

@@ -269,7 +269,7 @@ template <int V, int THR, typename F> __device__ __forceinline__ void with_colum
 template <typename T, int V, int THR, int ORDER>
 __global__ void __launch_bounds__(THR) fold_rmsnorm_rows_kernel(FoldArgs a) {
     sb::pdl_launch_dependents();
-    __shared__ float slot[2][stands_for<ORDER, V, THR>() * THR / 32];
+    __shared__ __align__(16) float slot[2][stands_for<ORDER, V, THR>() * THR / 32];
     const int m = blockIdx.x, d4 = a.d / 4, tid = threadIdx.x;
     sb::pdl_wait();
     const int r = a.row_index ? a.row_index[m] : m;
