@@ -37,4 +37,26 @@ __device__ __forceinline__ void tile_step(unsigned long long (&acc)[4][4 * NC], 
     }
 }
 
+// tile_step for a y that rows `from` and later of a group of four take: of the first group (PAIR0 0, the second takes it whole) or
+// of the second (PAIR0 2).  The others, whose x is zero, get a zero for it, whatever y is.
+template <int NC, int PAIR0>
+__device__ __forceinline__ void tile_step_from(unsigned long long (&acc)[4][4 * NC], const float* x, const float* y, int from) {
+    unsigned long long xs[4];
+    if (PAIR0 == 0) *reinterpret_cast<ulonglong2*>(xs) = *reinterpret_cast<const ulonglong2*>(x);
+    *reinterpret_cast<ulonglong2*>(xs + 2) = *reinterpret_cast<const ulonglong2*>(x + 32);
+#pragma unroll
+    for (int h = 0; h < NC; ++h) {
+        const float4 v = *reinterpret_cast<const float4*>(y + 64 * h);
+        const float ys[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const unsigned long long yy = twice(ys[j]);
+            fma2(acc[PAIR0][4 * h + j], xs[PAIR0], pair(from <= 0 ? ys[j] : 0.f, from <= 1 ? ys[j] : 0.f));
+            fma2(acc[PAIR0 + 1][4 * h + j], xs[PAIR0 + 1], pair(from <= 2 ? ys[j] : 0.f, from <= 3 ? ys[j] : 0.f));
+#pragma unroll
+            for (int p = PAIR0 + 2; p < 4; ++p) fma2(acc[p][4 * h + j], xs[p], yy);
+        }
+    }
+}
+
 }  // namespace sb

@@ -299,19 +299,22 @@ __global__ void __launch_bounds__(256) retention_chunk_kernel(RetChunkArgs ca) {
                     for (int k = 0; k < TB; ++k) inter[k][jj] = fmaf(qi[k], sv, inter[k][jj]);
                 }
             }
-            const int last = tk[TB - 1];
-            for (int s = 0; s <= last; ++s) {
-                float w[TB];
+            // a token's own and earlier values alone (a later one times a weight of zero is no zero where it is not finite)
+            int s = 0;
 #pragma unroll
-                for (int k = 0; k < TB; ++k) w[k] = As[tk[k] * C + s];
+            for (int k0 = 0; k0 < TB; ++k0)
+                for (; s <= tk[k0]; ++s) {
+                    float w[TB];
 #pragma unroll
-                for (int jj = 0; jj < JJ; ++jj) {
-                    const int j = lane + 32 * jj;
-                    const float vv = j < dv ? Vs[s * dv + j] : 0.f;
+                    for (int k = k0; k < TB; ++k) w[k] = As[tk[k] * C + s];
 #pragma unroll
-                    for (int k = 0; k < TB; ++k) acc[k][jj] = fmaf(w[k], vv, acc[k][jj]);
+                    for (int jj = 0; jj < JJ; ++jj) {
+                        const int j = lane + 32 * jj;
+                        const float vv = j < dv ? Vs[s * dv + j] : 0.f;
+#pragma unroll
+                        for (int k = k0; k < TB; ++k) acc[k][jj] = fmaf(w[k], vv, acc[k][jj]);
+                    }
                 }
-            }
 #pragma unroll
             for (int k = 0; k < TB; ++k) {
                 const int t = t0 + 8 * k;
@@ -461,10 +464,11 @@ int launch_retention_chunked(const RetArgs& a, int R, int C, int chunks, float* 
 // the kernels above is a shared-memory load per four multiply-adds.  Here a thread holds 8 x 8 outputs (tokens or state rows by
 // value columns; two-wide multiply-adds over pairs of tokens), so that four 16-byte loads feed 32 of them, and the operand
 // whose rows are contracted lies transposed (Qt, Kt, At: [contraction][token]).  V takes the state's place in shared memory once
-// Q S0 is done, which leaves room for three blocks an SM at 64 x 128.  Scores above the diagonal are zeros; the products of
-// the chunk's first 32 tokens with its last 32 values are left out.
-// The three launches (bfloat16, 16 heads): 1,500 tokens, 64 x 128: 151 us with the kernels above, 70 with these; 2,048 tokens
-// 180 / 89, 128 x 256 798 / 281, 32 x 64 90 / 48; 200 tokens of 64 x 128 83 / 55.
+// Q S0 is done, which leaves room for three blocks an SM at 64 x 128.  A token adds its own and earlier values alone: a warp's
+// tokens lie in two runs of eight, so a value is added by a whole run, by none of it, or (eight values a run) by some of it.
+// (Zero weights for the later values cost 1 to 2 % less, but a value that is not finite then reaches earlier tokens.)
+// The three launches (bfloat16, 16 heads): 1,500 tokens, 64 x 128: 151 us with the kernels above, 68 with these; 2,048 tokens
+// 180 / 90, 128 x 256 798 / 285, 32 x 64 90 / 46; 200 tokens of 64 x 128 83 / 55.
 constexpr int TC = 64;                  // tokens of a chunk
 constexpr int TPAD = TC + 4;            // floats between the rows of Qt, Kt and At
 
@@ -702,11 +706,16 @@ __global__ void __launch_bounds__(128 * COLS, COLS == 1 ? 3 : 1) retention_tiles
             }
         }
         __syncthreads();
-        // ---- and the chunk's own tokens
+        // ---- and the chunk's own tokens: the warp's are t0 .. t0 + 7 and those 32 on
+        const int t0 = 8 * ((tid >> 5) & 3);
 #pragma unroll 4
-        for (int s = 0; s < TC / 2; ++s) tile_step<NC, 0>(acc, Ks + s * TPAD + 4 * ty, SV + s * DV + col);
+        for (int s = 0; s < t0; ++s) tile_step<NC, 0>(acc, Ks + s * TPAD + 4 * ty, SV + s * DV + col);
 #pragma unroll 4
-        for (int s = TC / 2; s < TC; ++s) tile_step<NC, 2>(acc, Ks + s * TPAD + 4 * ty, SV + s * DV + col);
+        for (int s = t0; s < t0 + 8; ++s) tile_step_from<NC, 0>(acc, Ks + s * TPAD + 4 * ty, SV + s * DV + col, s - 4 * ty);
+#pragma unroll 4
+        for (int s = t0 + 8; s < t0 + 32; ++s) tile_step<NC, 2>(acc, Ks + s * TPAD + 4 * ty, SV + s * DV + col);
+#pragma unroll 4
+        for (int s = t0 + 32; s < t0 + 40; ++s) tile_step_from<NC, 2>(acc, Ks + s * TPAD + 4 * ty, SV + s * DV + col, s - 32 - 4 * ty);
         // ---- norm over the head, gate, store
         float ss[8];
 #pragma unroll

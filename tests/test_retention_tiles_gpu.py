@@ -70,3 +70,32 @@ def test_tiles(ops, dtype, dk, dv, turns, lengths):
     for tiles, other in zip(*errors):
         assert tiles <= 16 * 2.0 ** -24 + (2.0 ** -9 if dtype == torch.bfloat16 else 0), errors
         assert tiles <= 1.5 * other + 2.0 ** -23, errors
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("dk,dv", [(64, 128), (32, 256), (96, 64)])
+@pytest.mark.parametrize("at", [1, 7, 8, 37, 63, 64, 100])
+def test_a_value_that_is_not_finite_reaches_no_earlier_token(ops, dtype, dk, dv, at):
+    """An infinity among token `at`'s values: the tokens before it have the bits that they have without it, in the tile kernels
+    and (rows off 16 bytes) in the kernels for other heads, with chunks as launches and with one block a request."""
+    H, N = 3, 150
+    g = torch.Generator(device=DEV).manual_seed(at)
+    wide = torch.randn(N, 2 * H * (dk + dv), device=DEV, generator=g).to(dtype)
+    decay = torch.tensor([0.97, 0.995, 0.9995], device=DEV)
+    freq = 1.0 / 1e4 ** (torch.arange(0, dk, 2, device=DEV).double() / dk)
+    seq = [torch.tensor(t, dtype=torch.int32, device=DEV) for t in ([0, N], [0], [0])]
+    lent = torch.empty(ops.retention_scratch_size(N, 1, H, dk, dv), device=DEV)
+    for shift, scratch in ((0, lent), (1, lent), (1, None)):
+        outs = []
+        for value in (None, float("inf")):
+            buf = torch.empty(N * wide.shape[1] + shift, dtype=dtype, device=DEV)[shift:].view(wide.shape)
+            buf.copy_(wide)
+            if value is not None:
+                buf[at, 2 * H * dk + dv + 5] = value            # head 1
+            out = torch.full((N, H * dv), float("nan"), device=DEV, dtype=dtype)
+            ops.retention(out, buf, (0, H * dk, 2 * H * dk, 2 * H * dk + H * dv), torch.zeros(1, H, dk, dv, device=DEV), decay,
+                          freq.float(), dk, *seq, 1e-5, dk ** -0.5, chunked=True, inv_freq_lo=(freq - freq.float().double()).float(),
+                          scratch=scratch)
+            outs.append(out)
+        assert torch.equal(outs[0][:at], outs[1][:at]), (shift, scratch is not None)
+        assert not bool(torch.isfinite(outs[1][at, dv:2 * dv]).all())
