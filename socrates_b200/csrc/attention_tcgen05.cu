@@ -297,7 +297,8 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_k, const __g
     }
     sb::pdl_launch_dependents();
     // q and the pages are written by earlier kernels; the step's offsets, rows, positions and block table too, unless the
-    // caller says that they are older than the kernel before this one (three round trips to memory less after the wait).
+    // caller says that they were complete before the kernel before this one started (three round trips to memory less after
+    // the wait).  That kernel, and any number before it, may still be running here: none of them may write these arrays.
     // A prompt of 187 tokens through 18 layers 2,497 -> 2,434 us, one of 2,048 as before (its tiles hide the start).
     if (!meta_older) sb::pdl_wait();
 
@@ -790,7 +791,8 @@ extern "C" int sb_attention_tcgen05_pages_supports(int num_pages, int Hkv, int p
 // and ungated instead of to `out`; `cap`, `slopes` [Hq] and `chunk` as in score_map.cuh (0 / null: none);
 // `skip_single`: requests that bring one token are left out (their rows of the output are not written); `dist_bias`
 // [Hq, bias_len] (or null): added to the score of the key at distance min(d, bias_len - 1) after the cap; `meta_older`: the block
-// table and the seq_ arrays are older than the kernel before this one on the stream.
+// table and the seq_ arrays are complete before the kernel before this one on the stream starts (written by a copy, or by a
+// kernel that had ended before the first of the kernels launched dependently of one another started; by none of these).
 extern "C" int sb_attention_prefill_tcgen05(void* out, const void* q, const void* k_pool, const void* v_pool,
                                             int num_pages, const int* block_table, int table_width,
                                             const int* seq_starts, const int* seq_rows,

@@ -550,8 +550,10 @@ def attention_prefill_tcgen05(out: torch.Tensor, q: torch.Tensor, k_pool: torch.
     `softcap`, `slopes`, `chunk` as in `attention_decode_mma`.  `skip_single`: requests that bring one
     token are left out (see `attention_decode_balanced`); their rows of `out` are not written.  `dist_bias`
     float32 [Hq, L]: joins the score of the key at distance min(d, L - 1), after the cap.  `meta_older`: the block
-    table and the seq_ tensors are older than the kernel before this one on the stream (in a step they are: they
-    come with its one host copy), so they are read before that kernel has ended."""
+    table and the seq_ tensors are complete before the kernel before this one STARTS, so they are read before it has
+    ended.  Kernels of a chain let their successors start before their own wait, so a kernel two or more places back may
+    still be running: none of the chain may write them.  In a step they come by host copies ahead of its first
+    kernel, which waits for them."""
     N = q.shape[0]
     pages, Hkv, BS, D = k_pool.shape
     R = seq_rows.numel()
