@@ -939,3 +939,12 @@ int gemm_tcgen05_many_rows(const void* A, const void* W, void* C, int M, int N, 
                               : many_rows<float>(A, W, C, M, N, K, status, variant, epi, stream);
 }
 }  // namespace sb
+
+// The tile width that the persistent kernel takes for M x N when it is not told one (host only).
+extern "C" int sb_gemm_tcgen05_tile_width(int M, int N) {
+    if (M <= 0 || N <= 0) return 0;
+    int dev = 0, num_sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+    return pick_bn(M, N, num_sms);
+}

@@ -306,6 +306,11 @@ def gemm_tcgen05_shares_parts(M: int, N: int, K: int) -> int:
     return int(library().sb_gemm_tcgen05_shares_parts(int(M), int(N), int(K)))
 
 
+def gemm_tcgen05_tile_width(M: int, N: int) -> int:
+    """Columns of the tiles in which the persistent kernel takes a product of M rows (fewer than 4,096) by N columns."""
+    return int(library().sb_gemm_tcgen05_tile_width(int(M), int(N)))
+
+
 def gemm_tcgen05(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, status: torch.Tensor,
                  splits: int = 1, variant: int = 0, epilogue: int = 0,
                  prefetch: Optional[Tuple[torch.Tensor, int]] = None) -> int:

@@ -132,3 +132,28 @@ def test_fold_rmsnorm_rows_have_the_other_kernels_bits(ops, d, M, form):
         ops.fold_rmsnorm(r, delta, gain, out, EPS, **kw)
         sides.append((r, out.to(torch.bfloat16)))
     assert torch.equal(sides[0][0], sides[1][0]) and torch.equal(sides[0][1], sides[1][1])
+
+
+ACTIVATIONS = {"identity": lambda x: x, "relu_squared": lambda x: x.clamp(min=0) ** 2, "silu": torch.nn.functional.silu,
+               "gelu_tanh": lambda x: torch.nn.functional.gelu(x, approximate="tanh"), "tanh": torch.tanh}
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("act", list(ACTIVATIONS))
+@pytest.mark.parametrize("S,bias", [(0, True), (3, True), (1, False)])
+@pytest.mark.parametrize("N,F", [(3101, 424), (30, 424), (3101, 427)])
+def test_bias_act_against_64_bits(ops, dtype, act, S, bias, N, F):
+    """By 16 bytes (many values in rows of whole pieces) and a value at a time."""
+    g = torch.Generator(device=DEV).manual_seed(N + F)
+    x = torch.randn(S, N, F, device=DEV, generator=g) if S else torch.randn(N, F, device=DEV, generator=g).to(dtype)
+    b = torch.randn(F, device=DEV, generator=g) if bias else None
+    out = torch.full((N, F), float("nan"), device=DEV, dtype=dtype)
+    ops.bias_act(out, x, b, act)
+    terms = (x.double().abs().sum(0) if S else x.double().abs()) + (b.double().abs() if bias else 0)
+    z = (x.double().sum(0) if S else x.double()) + (b.double() if bias else 0)
+    want = ACTIVATIONS[act](z)
+    # S + 1 float32 additions, an activation whose slope is at most 2 |z| + 1.2 and which itself takes some ten roundings of
+    # numbers up to 1 + |z| + z^2, then the result's own rounding
+    bound = 2.0 ** -24 * ((S + 1) * terms * (2 * z.abs() + 1.2) + 16 * (1 + z.abs() + z * z)) + \
+        (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23) * want.abs()
+    assert bool(((out.double() - want).abs() <= bound).all())
