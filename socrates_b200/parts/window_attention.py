@@ -121,7 +121,7 @@ class WindowBiasAttention(Part):
         tail = cache.state("conv") if self.taps > 1 else None
         ops.short_conv(qkvg, self.in_bias, self.conv, None, False, tail, ctx.token_rows, ctx.positions,
                        [(0, self.Cq, q), (self.Cq, self.Cq + self.Ck, k_pool), (self.Cq + self.Ck, self.C, v_pool)],
-                       table, requests=ctx.num_seqs)
+                       table, ctx.num_seqs)
         if tail is not None:
             ops.short_conv_tail(tail, qkvg, self.in_bias, self.taps, ctx.seq_starts, ctx.seq_rows)
         attn = ctx.buffers.take("wa_attn", N, (self.H * self.dv,), ctx.dtype)
