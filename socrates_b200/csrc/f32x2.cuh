@@ -1,4 +1,5 @@
-// Two-wide float32 arithmetic and the register-tile step that the float32 kernels share.
+// Two-wide float32 arithmetic (retention and selective scan; gemm_f32.cu and linear_recurrence.cu have their own forms) and the
+// register-tile steps of the retention kernels.
 #pragma once
 
 #include <stdint.h>

@@ -474,8 +474,8 @@ int dispatch(const void* A, const void* W, void* C, int M, int N, int K, int spl
 // *splits_io: wanted number of K parts in, number actually written out (never more).
 // status: device int the kernel writes a non-zero code to if a bounded wait gave up.
 // variant: 0 = the kernels chosen by shape; 4 = one tile per block also for many rows
-//          (the default there is the persistent kernel); 128, 160, 256 = that tile width
-//          in the persistent kernel instead of the one it would choose; 1128, 1160, 1192,
+//          (the default there is the persistent kernel); 128, 160, 256, 288, 352, 416 = that tile
+//          width in the persistent kernel instead of the one it would choose; 1128, 1160, 1192,
 //          1256 = the pair kernel (two SMs per tile, cta_group::2) with tiles 256 x (variant - 1000);
 //          5 = the weight-streaming kernel for more than 64 rows (StepContext.wide_splits says where it pays);
 //          2000 = the pair kernel dealing equal shares of K blocks, float32 partial sums

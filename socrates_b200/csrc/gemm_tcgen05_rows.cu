@@ -28,7 +28,10 @@ namespace {
 // columns, a tile's main loop waits for the epilogue of the tile before it.
 //
 // BN > 256 (always two issuers, one accumulator): a product is at most 256 columns wide, so one warp issues the first half of
-// the columns and the other the rest, and the W tile comes as two boxes.
+// the columns and the other the rest, and the W tile comes as two boxes.  A sum is one chain, as with 256 columns, and has those
+// bits; with 128 and 160 columns each half of a K block has a chain of its own, and the tensor core cuts a chain's sum off at every
+// addition (2-norm against 64 bits, N(0,1) by N(0,0.02): K of 4,096 2.1e-6 with two chains, 4.4e-6 with one; of 8,192 4.4e-6 and
+// 9.1e-6; the bfloat16 operands are rounded at 1e-3).
 // Shared memory sets the pace (A is read once for each half), 0.475 us a K block at 288 columns for 0.36 at 256: they are for
 // products that then need one wave for two (pick_bn).
 constexpr int ACC_STRIDE = 256;          // TMEM columns between the two accumulators
@@ -789,7 +792,8 @@ constexpr int persistent_stages(int bn) {
 // Wider tiles (288 / 352 / 416 columns: 1,040 / 1,190 / 1,350 in the units below) where all are ONE wave, which has no epilogue
 // beside it, and eight row tiles or more share each panel of W: 2,048 x 2,560 x 9,728 80 us (160 columns 96, 256 115), x 4,096
 // 37 (45, 51), 1,024 x 6,144 x 2,560 30 (47, 38).  With two or three row tiles W's bytes set the pace and they lose: 187 x 19,456 x
-// 2,560 49 us (160 columns 45), 384 rows 64 (60).  A prompt of 1,023 tokens through 18 layers of 4B 5,287 -> 5,185 us.
+// 2,560 49 us (160 columns 45), 384 rows 64 (60).  Where 160 columns were the choice the sums' chains change with the width: 4,096 x
+// 12,288 1,200 rows 119.6 -> 106.5 us, 5,120 x 25,600 1,000 rows 247 -> 209.  A prompt of 1,023 tokens through 18 layers of 4B 5,287 -> 5,185 us.
 static int pick_bn(int M, int N, int num_sms) {
     const int tiles_m = (M + BM - 1) / BM;
     int best = 256;

@@ -235,7 +235,15 @@ class StepContext:
         float32).  Measured, equal shares / the best whole tiles (us): 2,560 x 9,728: 640 rows 42.3 / 40.1, 1,023 50.9 / 45.0,
         1,280 58.7 / 62.2, 1,500 71.3 / 63.2, 2,048 89.1 / 98.6; 2,560 x 4,096: 1,023 32.3 / 21.0, 2,048 45.4 / 44.9; 4,096 x 4,096:
         512 26.5 / 19.8, 1,023 36.9 / 29.7, 1,280 42.1 / 44.9, 1,500 47.6 / 52.2, 1,792 53.3 / 52.6; 5,120 x 8,192: 512 48.1 / 41.9,
-        1,023 74.4 / 85.3."""
+        1,023 74.4 / 85.3.
+
+        Whole tiles have to be 2 % cheaper by these fits to be taken: where the two come out alike (they are wrong by up to 8 %)
+        the kernel stays that ran before the fits, so that no prompt's bits move for nothing.  The costs leave out the widths
+        beyond 256, which whole tiles take where they are one wave and eight row tiles: with the norm behind it, equal shares /
+        288 columns, 2,048 rows of 2,560 x 4,096 62.0 / 48.6 us, of 2,560 x 9,728 102.7 / 92.5.  Which sums the K blocks of a
+        product are cut into differs, too (2-norm against 64 bits at K of 4,096: equal shares 1.5e-6 to 3.7e-6, whole tiles of 128
+        and 160 columns 2.1e-6, wider 4.4e-6; in proportion to K beyond); the next norm rounds to bfloat16, at 1e-3, and
+        logits are as far from 64 bits either way (4B, 520 to 1,500 tokens: 0.018 to 0.020 both)."""
         parts = self._shares_parts(M, w, x_dtype)
         return parts if parts and self._shares_pay(M, w) else 0
 
