@@ -835,7 +835,7 @@ extern "C" int sb_retention(const void* qkvg, long long stride, int q_off, int k
             const bool spread = scratch != nullptr && R * H < 132 && chunks > 2 * R &&
                                 (long long)chunks * H * dk * dv <= scratch_floats;
             const int tiles = (N + TC - 1) / TC + R;        // (the tile kernels' chunks, never more than the others')
-            if (spread && tiles_take(a, scratch, dtype == SB_F32 ? 4 : 2)) {
+            if (spread && (dtype == SB_F32 || dtype == SB_BF16) && tiles_take(a, scratch, dtype == SB_F32 ? 4 : 2)) {
                 if (dtype == SB_F32) launch_retention_tiles<float>(a, R, tiles, scratch, stream);
                 else launch_retention_tiles<__nv_bfloat16>(a, R, tiles, scratch, stream);
                 SB_LAUNCH_CHECK();

@@ -99,3 +99,18 @@ def test_a_value_that_is_not_finite_reaches_no_earlier_token(ops, dtype, dk, dv,
             outs.append(out)
         assert torch.equal(outs[0][:at], outs[1][:at]), (shift, scratch is not None)
         assert not bool(torch.isfinite(outs[1][at, dv:2 * dv]).all())
+
+
+@pytest.mark.parametrize("lent", [False, True])
+def test_an_element_type_that_no_kernel_has_is_refused(ops, monkeypatch, lent):
+    H, dk, dv, N = 2, 64, 128, 300
+    x = torch.randn(N, 2 * H * (dk + dv), device=DEV).to(torch.bfloat16)
+    seq = [torch.tensor(t, dtype=torch.int32, device=DEV) for t in ([0, N], [0], [0])]
+    scratch = torch.empty(ops.retention_scratch_size(N, 1, H, dk, dv), device=DEV) if lent else None
+    out = torch.full((N, H * dv), 7.0, device=DEV, dtype=torch.bfloat16)
+    monkeypatch.setattr(ops, "_code", lambda dtype: 2)
+    with pytest.raises(ops.KernelError, match="dtype 2"):
+        ops.retention(out, x, (0, H * dk, 2 * H * dk, 2 * H * dk + H * dv), torch.zeros(1, H, dk, dv, device=DEV),
+                      torch.full((H,), 0.9, device=DEV), torch.ones(dk // 2, device=DEV), 0, *seq, 1e-5, 1.0, chunked=True,
+                      scratch=scratch)
+    assert bool((out == 7.0).all())
